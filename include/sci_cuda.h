@@ -318,13 +318,13 @@ typedef struct sci_solve_items {
     int32_t *iterations;           /* refinement iterations per system, or null            */
 } sci_solve_items;
 typedef struct sci_cuda_solve_batch sci_cuda_solve_batch;
-/* Checks every system, tunes the block size of each order bucket (<= 32, <= 64, <= 128, <= 256;
- * cached like the chunk batches), and captures one launch per bucket into a CUDA graph. The tuning
- * launches solve the systems. Waits. */
+/* Checks every system, groups the systems by order and captures the groups' launches into a CUDA
+ * graph. Waits. */
 int sci_cuda_solve_batch_create(sci_cuda_context *context, const sci_solve_items *items, sci_cuda_solve_batch **batch);
 /* Replays the graph on the context's stream (queued). */
 int sci_cuda_solve_batch_launch(sci_cuda_solve_batch *batch);
-/* Threads per CTA chosen for each bucket (0: the bucket is empty). */
+/* Threads per CTA, one per row, of the largest launch in each order bucket (<= 32, <= 64, <= 128,
+ * <= 256; 0: the bucket is empty). */
 int sci_cuda_solve_batch_shapes(const sci_cuda_solve_batch *batch, uint32_t *threads);
 /* Waits for the context's queued work, then frees the batch. */
 int sci_cuda_solve_batch_destroy(sci_cuda_solve_batch *batch);

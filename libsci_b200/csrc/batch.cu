@@ -14,7 +14,8 @@
 // $HOME/.cache/sci_cuda/batch_tune.txt) that later processes read; SCI_CUDA_TUNE=0 skips tuning.
 #include "batch_kernel.cuh"
 #include "context.hpp"
-#include "solve_batch_kernel.cuh"
+#include "small_solve.cuh"
+#include "small_solve.hpp"
 #include "specialize.hpp"
 
 #include <cuda_runtime.h>
@@ -406,55 +407,37 @@ extern "C" int sci_cuda_batch_destroy(sci_cuda_batch *batch) {
 
 // ---- batched small solves ---------------------------------------------------------------------
 // Thousands of independent systems (n <= 256, one right-hand side, double operands), FP32 LU and
-// FP64 refinement inside one CTA per system (solve_batch_kernel.cuh). Systems are grouped into four
-// buckets by order (<= 32, <= 64, <= 128, <= 256); each bucket is one launch whose block size the
-// autotuner picks among the variants that fit it (timed on the bucket's own systems, cached like
-// the chunk batches' spans). The four launches are captured into one CUDA graph on parallel
-// branches, so small buckets fill the gaps of the large one.
+// FP64 refinement inside one CTA per system (small_solve.cuh). Systems are grouped by order; each
+// group is one launch of a thread per row of its largest system, and the launches are captured into
+// one CUDA graph on parallel branches, the largest orders first, so small systems fill the gaps that
+// large ones leave.
+
+namespace {
+
+    // The groups' largest orders: where another system fits beside it on an SM (shared memory: eight of
+    // order 64, four of 96, three of 128, two of 152, one above), and every 32 rows beyond, where a
+    // group's warps all have rows. The last bound of each reported bucket (<= 32, <= 64, <= 128, <= 256).
+    constexpr int kGroups = 8;
+    constexpr unsigned kGroupLimit[kGroups] = {32, 64, 96, 128, 152, 192, 224, 256};
+    constexpr int kGroupBucket[kGroups] = {0, 1, 2, 2, 3, 3, 3, 3};
+
+    int solve_group(unsigned n) {
+        int g = 0;
+        while (n > kGroupLimit[g]) ++g;
+        return g;
+    }
+
+} // namespace
 
 struct sci_cuda_solve_batch {
     sci_cuda_context *context{nullptr};
     void *memory{nullptr};
     unsigned threads[4]{};
-    cudaStream_t branches[4]{};
-    cudaEvent_t fork{nullptr}, joins[4]{};
+    cudaStream_t branches[kGroups]{};
+    cudaEvent_t fork{nullptr}, joins[kGroups]{};
     cudaGraph_t graph{nullptr};
     cudaGraphExec_t exec{nullptr};
 };
-
-namespace {
-
-    struct Variant {
-        int threads, rc;
-        const void *kernel;
-    };
-    const Variant kVariants[] = {
-            {32, 0, reinterpret_cast<const void *>(&small_solve<32, 0>)},
-            {64, 0, reinterpret_cast<const void *>(&small_solve<64, 0>)},
-            {128, 0, reinterpret_cast<const void *>(&small_solve<128, 0>)},
-            {256, 0, reinterpret_cast<const void *>(&small_solve<256, 0>)},
-            {256, kSmallRegisters, reinterpret_cast<const void *>(&small_solve<256, kSmallRegisters>)},
-            {512, kSmallRegisters, reinterpret_cast<const void *>(&small_solve<512, kSmallRegisters>)},
-    };
-
-    int solve_bucket(unsigned n) { return n <= 32 ? 0 : (n <= 64 ? 1 : (n <= 128 ? 2 : 3)); }
-
-    // The variants that may run a bucket whose largest order is `most`.
-    std::vector<const Variant *> candidates(int bucket, unsigned most) {
-        std::vector<const Variant *> out;
-        for (const Variant &v : kVariants) {
-            const bool registers = v.rc > 0;
-            if (bucket < 3 && registers) continue;
-            if (bucket == 3 && most > kSmallShared && !registers) continue;  // only the register form fits
-            if (registers && static_cast<unsigned>(v.threads) < most) continue;
-            if (bucket == 0 && v.threads > 128) continue;
-            if (bucket >= 2 && v.threads < 64) continue;
-            out.push_back(&v);
-        }
-        return out;
-    }
-
-} // namespace
 
 extern "C" int sci_cuda_solve_batch_create(sci_cuda_context *context, const sci_solve_items *items,
                                            sci_cuda_solve_batch **batch) {
@@ -467,20 +450,20 @@ extern "C" int sci_cuda_solve_batch_create(sci_cuda_context *context, const sci_
     cudaSetDevice(ctx.device);
     const unsigned count = items->systems;
     std::vector<SmallSystem> systems(count);
-    std::vector<unsigned> lists[4];
-    unsigned most[4] = {};
+    std::vector<unsigned> lists[kGroups];
+    unsigned most[kGroups] = {};
     for (unsigned s = 0; s < count; ++s) {
         const unsigned n = items->orders[s];
-        if (n == 0 || n > static_cast<unsigned>(kSmallMax))
-            return ctx.fail(SCI_CUDA_ERROR_UNSUPPORTED, "system %u: order %u outside 1..%d", s, n, kSmallMax);
+        if (n == 0 || n > kSmallOrder)
+            return ctx.fail(SCI_CUDA_ERROR_UNSUPPORTED, "system %u: order %u outside 1..%llu", s, n, kSmallOrder);
         const void *a = items->matrices[s], *b = items->rights[s];
         void *x = items->solutions[s];
         if (!a || !b || !x || !reachable(ctx, a) || !reachable(ctx, b) || !reachable(ctx, x))
             return ctx.fail(SCI_CUDA_ERROR_INVALID, "system %u: an operand is not memory of this device", s);
-        systems[s] = SmallSystem{static_cast<const double *>(a), static_cast<const double *>(b), static_cast<double *>(x), n, 0};
-        const int b_ = solve_bucket(n);
-        lists[b_].push_back(s);
-        most[b_] = std::max(most[b_], n);
+        systems[s] = SmallSystem{static_cast<const double *>(a), static_cast<const double *>(b), static_cast<double *>(x), n, 1, 1, 0};
+        const int g = solve_group(n);
+        lists[g].push_back(s);
+        most[g] = std::max(most[g], n);
     }
     if ((items->errors && !reachable(ctx, items->errors)) || (items->iterations && !reachable(ctx, items->iterations)))
         return ctx.fail(SCI_CUDA_ERROR_INVALID, "errors / iterations are not memory of this device");
@@ -500,98 +483,34 @@ extern "C" int sci_cuda_solve_batch_create(sci_cuda_context *context, const sci_
     };
     auto *device_systems = static_cast<SmallSystem *>(made->memory);
     auto *device_order = reinterpret_cast<unsigned *>(static_cast<unsigned char *>(made->memory) + table);
-    unsigned offsets[4] = {};
+    unsigned offsets[kGroups] = {};
     std::vector<unsigned> flat;
-    for (int b = 0; b < 4; ++b) {
-        offsets[b] = static_cast<unsigned>(flat.size());
-        flat.insert(flat.end(), lists[b].begin(), lists[b].end());
+    for (int g = 0; g < kGroups; ++g) {
+        offsets[g] = static_cast<unsigned>(flat.size());
+        flat.insert(flat.end(), lists[g].begin(), lists[g].end());
+        if (!lists[g].empty()) made->threads[kGroupBucket[g]] = (most[g] + 31) / 32 * 32;
     }
     cudaMemcpyAsync(device_systems, systems.data(), count * sizeof(SmallSystem), cudaMemcpyHostToDevice, ctx.stream);
     cudaMemcpyAsync(device_order, flat.data(), flat.size() * 4, cudaMemcpyHostToDevice, ctx.stream);
     if (int code = ctx.check(cudaStreamSynchronize(ctx.stream), "uploading the system tables")) return fail(code);
 
-    double *errors = items->errors;
-    int *iterations = items->iterations;
-    auto launch = [&](int b, const Variant &v, cudaStream_t stream) -> int {
-        const unsigned long long smem = small_shared_bytes(most[b], v.rc);
-        if (smem > ctx.shared_limit) return ctx.fail(SCI_CUDA_ERROR_UNSUPPORTED, "bucket %d needs %llu bytes of shared memory", b, smem);
-        cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        const unsigned *order = device_order + offsets[b];
-        void *args[] = {&device_systems, &order, &errors, &iterations};
-        return ctx.check(cudaLaunchKernel(v.kernel, dim3(static_cast<unsigned>(lists[b].size())), dim3(v.threads), args, smem, stream),
-                         "launching a batch of small solves");
-    };
-
-    // tune each bucket's block size
-    const char *tune = std::getenv("SCI_CUDA_TUNE");
-    const bool tuning = !(tune && tune[0] == '0');
-    {
-        std::lock_guard<std::mutex> guard(cache_guard);
-        load_cache();
-    }
-    const Variant *chosen[4] = {};
-    for (int b = 0; b < 4; ++b) {
-        if (lists[b].empty()) continue;
-        const auto options = candidates(b, most[b]);
-        if (options.empty()) return fail(ctx.fail(SCI_CUDA_ERROR_UNSUPPORTED, "no variant for bucket %d", b));
-        chosen[b] = options.back();
-        std::string key;
-        for (char ch : ctx.name) key += (ch == ' ' ? '_' : ch);
-        key += "|solve|" + std::to_string(b);
-        if (!tuning) continue;
-        {
-            std::lock_guard<std::mutex> guard(cache_guard);
-            auto hit = cache.find(key);
-            if (hit != cache.end()) {
-                for (const Variant *v : options)
-                    if (static_cast<unsigned>(v->threads) == hit->second) chosen[b] = v;
-                continue;
-            }
-        }
-        float best = -1.0f;
-        for (const Variant *v : options) {
-            cudaEvent_t start, stop;
-            cudaEventCreate(&start);
-            cudaEventCreate(&stop);
-            std::vector<float> times;
-            for (int rep = 0; rep < 4; ++rep) {
-                cudaEventRecord(start, ctx.stream);
-                if (int code = launch(b, *v, ctx.stream)) return fail(code);
-                cudaEventRecord(stop, ctx.stream);
-                if (int code = ctx.check(cudaEventSynchronize(stop), "timing a solve variant")) return fail(code);
-                float ms = 0.0f;
-                cudaEventElapsedTime(&ms, start, stop);
-                if (rep > 0) times.push_back(ms);
-            }
-            cudaEventDestroy(start);
-            cudaEventDestroy(stop);
-            std::sort(times.begin(), times.end());
-            if (best < 0.0f || times[1] < best) {
-                best = times[1];
-                chosen[b] = v;
-            }
-        }
-        std::lock_guard<std::mutex> guard(cache_guard);
-        store_cache(key, static_cast<unsigned>(chosen[b]->threads));
-    }
-    for (int b = 0; b < 4; ++b) made->threads[b] = chosen[b] ? static_cast<unsigned>(chosen[b]->threads) : 0u;
-
-    // capture: fork to one branch per bucket, join back
+    // capture: fork to one branch per group, join back
     cudaEventCreateWithFlags(&made->fork, cudaEventDisableTiming);
-    for (int b = 0; b < 4; ++b) {
-        cudaStreamCreateWithFlags(&made->branches[b], cudaStreamNonBlocking);
-        cudaEventCreateWithFlags(&made->joins[b], cudaEventDisableTiming);
+    for (int g = 0; g < kGroups; ++g) {
+        cudaStreamCreateWithFlags(&made->branches[g], cudaStreamNonBlocking);
+        cudaEventCreateWithFlags(&made->joins[g], cudaEventDisableTiming);
     }
     if (int code = ctx.check(cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal), "capturing the solves"))
         return fail(code);
     int launched = SCI_CUDA_OK;
     cudaEventRecord(made->fork, ctx.stream);
-    for (int b = 3; b >= 0 && !launched; --b) {
-        if (!chosen[b]) continue;
-        cudaStreamWaitEvent(made->branches[b], made->fork, 0);
-        launched = launch(b, *chosen[b], made->branches[b]);
-        cudaEventRecord(made->joins[b], made->branches[b]);
-        cudaStreamWaitEvent(ctx.stream, made->joins[b], 0);
+    for (int g = kGroups - 1; g >= 0 && !launched; --g) {
+        if (lists[g].empty()) continue;
+        cudaStreamWaitEvent(made->branches[g], made->fork, 0);
+        launched = small_solve_table(ctx, made->branches[g], device_systems, device_order + offsets[g],
+                                     static_cast<unsigned>(lists[g].size()), most[g], 1e-15, items->errors, items->iterations);
+        cudaEventRecord(made->joins[g], made->branches[g]);
+        cudaStreamWaitEvent(ctx.stream, made->joins[g], 0);
     }
     cudaGraph_t graph = nullptr;
     const cudaError_t ended = cudaStreamEndCapture(ctx.stream, &graph);
@@ -629,9 +548,9 @@ extern "C" int sci_cuda_solve_batch_destroy(sci_cuda_solve_batch *batch) {
         cudaStreamSynchronize(context->stream);
         if (batch->exec) cudaGraphExecDestroy(batch->exec);
         if (batch->graph) cudaGraphDestroy(batch->graph);
-        for (int b = 0; b < 4; ++b) {
-            if (batch->branches[b]) cudaStreamDestroy(batch->branches[b]);
-            if (batch->joins[b]) cudaEventDestroy(batch->joins[b]);
+        for (int g = 0; g < kGroups; ++g) {
+            if (batch->branches[g]) cudaStreamDestroy(batch->branches[g]);
+            if (batch->joins[g]) cudaEventDestroy(batch->joins[g]);
         }
         if (batch->fork) cudaEventDestroy(batch->fork);
         if (batch->memory) cudaFree(batch->memory);

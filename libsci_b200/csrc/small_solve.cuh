@@ -1,0 +1,920 @@
+// small_solve.cuh -- systems of order 256 or less, one CTA per system (and group of right-hand sides).
+//
+// A system (double operands) is factored in FP32 and refined in FP64 inside one CTA; nothing but its
+// matrix, right-hand sides and solution is in global memory. The CTA has a thread per row (32 threads
+// for each 32 rows), and a row stays where it was loaded, in its own row of shared memory, from the
+// load to the last substitution: a pivot exchange only changes the row's `place` (its position under
+// the reference's row exchanges), no value moves. The rows' pitch is an odd multiple of 16 bytes, so
+// eight rows' 16-byte pieces fall on all 32 banks. A system of more than kSmallWhole rows does not
+// fit; the entries of its last two 32-column blocks stay in the registers of the rows' threads.
+//
+// Factorisation, by 32-column blocks, left-looking: every earlier block K is applied to the block, and
+// the block is factored column by column.
+//  - applying block K: the 32 rows placed in it are published (shared memory); U_K = inv(L_KK) W_K is
+//    one small product by two warps; every row below subtracts L[row, K] U_K. A warp holds its 32
+//    rows' entries of the block as tiles of 4 rows x 8 columns per lane through all K (a row per
+//    lane reads 33 values for 32 multiplications, and shared memory returns a quarter of what the
+//    multipliers consume: 6.3 thousand cycles a step at order 256; the tile reads 12 for 32), a pair of columns per FMA
+//    instruction. Two barriers.
+//  - a column: two rows per thread, their entries of the block in registers. Each warp finds its largest
+//    |value| (the lowest place among equals: the first row with the strictly largest |a|,
+//    include/linear/decompose.hpp:29-72; a zero pivot skips the column's elimination); after a barrier
+//    every warp knows the pivot, its thread publishes the row, and after another every thread eliminates.
+//  - the block's triangles are inverted in place (a warp each for L and U), for the products above and
+//    for the substitutions.
+// Refinement: x = 0, r = b; repeat { d = U^-1 L^-1 P r in FP32; x += d; r = b - A x in FP64 } until the
+// normwise backward error |r|_inf / (|A|_inf |x|_inf + |b|_inf) is at most `target` or stops halving
+// (at most 30 corrections): the rule of sci_cuda_solve's refinement. A substitution step is a 32 x 32
+// product with the block's inverse by one warp and an update of the other rows from their own L or U.
+//
+// What bounds it: the chain of columns (700 cycles each at order 128, 790 at 256: two barriers, a
+// warp-wide maximum and vote, four trips through shared memory) and of barriers; systems of order 152
+// or less run several to an SM and fill each other's gaps. 4096 systems with orders uniform in
+// [8, 256]: 2.81 ms, where a column by column elimination in shared memory (about 3900 cycles a
+// column at 256) took 11.8 ms. One wave of 148 systems of order 64 / 128 / 256: 49 / 98 / 248 us.
+#pragma once
+
+#include "chunk_kernel.cuh"  // static_for
+
+namespace sci_cuda {
+
+    struct SmallSystem {
+        const double *a;  // n x n, row-major
+        const double *b;  // n rows of right-hand sides, `pitch` apart
+        double *x;        // laid out as b
+        unsigned n;
+        unsigned pitch;
+        unsigned columns;     // right-hand sides from b on that this CTA solves (at most the kernel's NR)
+        unsigned transposed;  // solve A^T x = b
+    };
+
+    constexpr int kSmallMax = 256;        // largest order
+    constexpr int kSmallWhole = 224;      // largest order whose factors lie in shared memory whole
+    constexpr int kSmallShared = 192;     // columns kept in shared memory beyond it (the other two blocks in registers)
+    constexpr int kSmallPitch = 36;       // floats between the rows of a 32 x 32 block apart from the matrix
+
+    // Floats between the matrix's rows: its columns, up to an odd number of 16-byte pieces.
+    __host__ __device__ inline int small_pitch(int n, int register_blocks) {
+        return 4 * (((register_blocks > 0 ? kSmallShared : n) + 3) / 4 | 1);
+    }
+
+    // Dynamic shared memory of one launch for systems up to order `most`.
+    inline unsigned long long small_shared_bytes(int most, int right_sides, int register_blocks) {
+        unsigned long long bytes = 4ull * most * small_pitch(most, register_blocks);  // factors
+        bytes += 2ull * 32 * kSmallPitch * 4;                    // published blocks (later: residuals)
+        bytes += 4ull * register_blocks * 32 * kSmallPitch;      // inverses of register blocks
+        bytes += 8ull * most * right_sides;                      // x
+        bytes += 2ull * 2 * most;                                // rows by position, positions by row
+        return (bytes + 15) / 16 * 16;
+    }
+
+    __device__ __forceinline__ unsigned long long small_pair(float lo, float hi) {
+        unsigned long long out;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(out) : "f"(lo), "f"(hi));
+        return out;
+    }
+    __device__ __forceinline__ void small_unpair(unsigned long long v, float &lo, float &hi) {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    }
+    // (lo, hi) += f * (u, v), each lane rounded once
+    __device__ __forceinline__ void small_fma_pair(float &lo, float &hi, unsigned long long f, float u, float v) {
+        unsigned long long out;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(out) : "l"(f), "l"(small_pair(u, v)), "l"(small_pair(lo, hi)));
+        small_unpair(out, lo, hi);
+    }
+
+    // Predicated stores to shared memory (two words, a 16-byte piece): no branch around them.
+    __device__ __forceinline__ void small_store_if(bool yes, void *to, unsigned a, unsigned b) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.v2.u32 [%1], {%2, %3};\n\t}" ::"r"(yes ? 1u : 0u),
+                     "r"(smem_address(to)), "r"(a), "r"(b)
+                     : "memory");
+    }
+    __device__ __forceinline__ void small_store_if(bool yes, void *to, float a, float b, float c, float d) {
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n\t}" ::"r"(
+                             yes ? 1u : 0u),
+                     "r"(smem_address(to)), "f"(a), "f"(b), "f"(c), "f"(d)
+                     : "memory");
+    }
+
+    __device__ __forceinline__ double small_larger(double v, double m) { return (v > m || v != v) ? v : m; }  // NaN wins
+
+    // Sums M values of every lane over the warp, M a power of two up to 8: lanes exchange halves of the
+    // values while they can, so value m's sum ends in the lanes whose top bits spell m.
+    template <int M> __device__ __forceinline__ double small_warp_sums(double (&s)[M], int lane, int &which) {
+        which = 0;
+        int offset = 16;
+#pragma unroll
+        for (int half = M / 2; half > 0; half /= 2, offset /= 2) {
+            const bool upper = (lane & offset) != 0;
+#pragma unroll
+            for (int m = 0; m < half; ++m) {
+                const double send = upper ? s[m] : s[m + half];
+                const double keep = upper ? s[m + half] : s[m];
+                s[m] = keep + __shfl_xor_sync(0xffffffffu, send, offset);
+            }
+            which += upper ? half : 0;
+        }
+        double total = s[0];
+#pragma unroll
+        for (; offset > 0; offset /= 2) total += __shfl_xor_sync(0xffffffffu, total, offset);
+        return total;
+    }
+
+    // One call's right-hand sides, `group` of them per CTA: CTAs [0, groups) solve A x = b, and with
+    // `b_transposed` CTAs [groups, 2 groups) solve A^T x = b_transposed.
+    struct SmallCall {
+        const double *a, *b, *b_transposed;
+        double *x, *x_transposed;
+        unsigned n, width, group, groups;
+        __device__ __forceinline__ SmallSystem system(unsigned block) const {
+            const bool flip = block >= groups;
+            const unsigned first = (flip ? block - groups : block) * group;
+            return SmallSystem{a, (flip ? b_transposed : b) + first, (flip ? x_transposed : x) + first, n, width,
+                               width - first < group ? width - first : group, flip ? 1u : 0u};
+        }
+    };
+
+    // NR: right-hand sides of a CTA. RB: 32-column blocks in registers (0, or 2 for n > kSmallWhole). The systems
+    // come from a table in device memory, the CTA's by `order`, or from `call` when there is no table.
+    template <int NR, int RB>
+    __global__ void __maxnreg__(RB > 0 ? 255 : 168)
+            small_solve(const SmallSystem *systems, const unsigned *order, const __grid_constant__ SmallCall call,
+                        double target, double *errors, int *iterations) {
+        constexpr int kWarps = kSmallMax / 32;
+        constexpr unsigned kAll = 0xffffffffu;
+        __shared__ __align__(16) float pivot_rows[2][32];      // the pivot's row of the block, by column parity
+        __shared__ __align__(8) float2 pivot_reciprocals[2];   // a scale and the scaled pivot's reciprocal
+        __shared__ __align__(16) uint2 best[kWarps];           // each warp's largest key (0: no row left) and its place
+        __shared__ __align__(16) float to_solve[32 * NR], solved[32 * NR];  // a substitution step's block, in and out
+        __shared__ double maxima[kWarps][2 * NR];
+        extern __shared__ __align__(16) unsigned char small_shared[];
+
+        const unsigned id = order ? order[blockIdx.x] : blockIdx.x;
+        const SmallSystem sys = systems ? systems[id] : call.system(blockIdx.x);
+        const int n = static_cast<int>(sys.n), nb = (n + 31) / 32, P = small_pitch(n, RB);
+        const int SB = RB > 0 ? kSmallShared / 32 : nb;        // blocks in shared memory
+        const int columns = RB > 0 ? kSmallShared : (n + 3) / 4 * 4;  // columns there, zeros beyond n
+        const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+        const bool row = tid < n;
+        const double *a = sys.a;
+
+        float *A = reinterpret_cast<float *>(small_shared);
+        unsigned char *cursor = small_shared + 4ull * n * P;
+        float *published = reinterpret_cast<float *>(cursor);  // the block's rows as they were
+        float *u_block = published + 32 * kSmallPitch;         // and as rows of U (or a block's L and U to invert)
+        double *r = reinterpret_cast<double *>(cursor);        // residuals, once the factors are done
+        cursor += 2ull * 32 * kSmallPitch * 4;
+        float *inverses = reinterpret_cast<float *>(cursor);
+        cursor += 4ull * RB * 32 * kSmallPitch;
+        double *x = reinterpret_cast<double *>(cursor);
+        unsigned short *rows = reinterpret_cast<unsigned short *>(x + n * NR);  // the row at each position
+        unsigned short *places = rows + n;                                      // each row's place
+        float *own = A + tid * P;
+        auto vector = [](float *p) -> float4 & { return *reinterpret_cast<float4 *>(p); };
+
+        // ---- load A in FP32, with |A|_inf
+        float held[RB > 0 ? RB : 1][32];
+        double norm = 0.0;  // the largest row sum this thread saw
+        if (sys.transposed) {
+            // row t of A^T is column t of A: a thread's loads are a warp's consecutive columns
+            if (row) {
+                const int stored = RB > 0 ? kSmallShared : n;
+#pragma unroll 16
+                for (int c = 0; c < stored; ++c) {
+                    const double v = a[1ll * c * n + tid];
+                    own[c] = static_cast<float>(v);
+                    norm += fabs(v);
+                }
+                for (int c = stored; c < columns; ++c) own[c] = 0.0f;
+                if constexpr (RB > 0) {
+#pragma unroll
+                    for (int q = 0; q < RB; ++q)
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) {
+                            const int at = kSmallShared + 32 * q + c;
+                            const double v = at < n ? a[1ll * at * n + tid] : 0.0;
+                            held[q][c] = static_cast<float>(v);
+                            norm += fabs(v);
+                        }
+                }
+            }
+        } else {
+            // a warp per row, the loads of several rows in flight: G pieces of 32 columns each
+            auto load = [&](auto g_c) {
+                constexpr int G = decltype(g_c)::value, R = G <= 4 ? 8 : 4;
+                for (int row0 = warp; row0 < n; row0 += R * warps) {
+                    double v[R][G], sum[R];
+#pragma unroll
+                    for (int u = 0; u < R; ++u)
+#pragma unroll
+                        for (int g = 0; g < G; ++g) {
+                            const int at = row0 + u * warps, c = lane + 32 * g;
+                            v[u][g] = at < n && c < n ? a[1ll * at * n + c] : 0.0;
+                        }
+#pragma unroll
+                    for (int u = 0; u < R; ++u) {
+                        const int at = row0 + u * warps;
+                        sum[u] = 0.0;
+#pragma unroll
+                        for (int g = 0; g < G; ++g) {
+                            const int c = lane + 32 * g;
+                            if (at < n && c < columns) A[at * P + c] = static_cast<float>(v[u][g]);
+                            sum[u] += fabs(v[u][g]);
+                        }
+                    }
+                    int which;
+                    norm = small_larger(small_warp_sums<R>(sum, lane, which), norm);
+                }
+            };
+            if (nb == 1) load(Int<1>{});
+            else if (nb == 2) load(Int<2>{});
+            else if (nb <= 4) load(Int<4>{});
+            else load(Int<8>{});
+            if constexpr (RB > 0) {
+#pragma unroll
+                for (int q = 0; q < RB; ++q)
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) {
+                        const int at = kSmallShared + 32 * q + c;
+                        held[q][c] = row && at < n ? static_cast<float>(a[1ll * tid * n + at]) : 0.0f;
+                    }
+            }
+        }
+        double rhs[NR], b_norm[NR], a_norm = 0.0;  // this thread's row of b, then |b_q|_inf and |A|_inf
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            rhs[q] = row && q < static_cast<int>(sys.columns) ? sys.b[1ull * tid * sys.pitch + q] : 0.0;
+            b_norm[q] = fabs(rhs[q]);
+        }
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1) {
+            norm = small_larger(__shfl_xor_sync(kAll, norm, offset), norm);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) b_norm[q] = small_larger(__shfl_xor_sync(kAll, b_norm[q], offset), b_norm[q]);
+        }
+        if (lane == 0) {
+            maxima[warp][0] = norm;
+#pragma unroll
+            for (int q = 0; q < NR; ++q) maxima[warp][NR + q] = b_norm[q];
+        }
+        if (row) {
+            places[tid] = static_cast<unsigned short>(tid);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) x[tid * NR + q] = 0.0;
+        }
+        for (int i = tid; i < 32 * NR; i += blockDim.x) to_solve[i] = 0.0f;
+        if (tid < kWarps) best[tid] = make_uint2(0u, ~0u);
+        __syncthreads();
+        for (int w = 0; w < warps; ++w) {
+            a_norm = small_larger(maxima[w][0], a_norm);
+#pragma unroll
+            for (int q = 0; q < NR; ++q) b_norm[q] = small_larger(maxima[w][NR + q], b_norm[q]);
+        }
+
+        // ---- LU with partial pivoting
+        int place = row ? tid : kSmallMax;
+        // row i of the inverse of block K's triangles (L's strictly below the diagonal, U's on and above it)
+        auto inverse_row = [&](int K, int i) -> float * {
+            if (RB > 0 && K >= SB) return inverses + ((K - SB) * 32 + i) * kSmallPitch;
+            return A + rows[32 * K + i] * P + 32 * K;
+        };
+        // U_K = inv(L_KK) W_K: 64 threads, four rows and four columns each
+        auto product = [&](int K) {
+            if (tid < 64) {
+                const int i0 = (tid >> 3) * 4, c = (tid & 7) * 4;
+                float4 acc[4];
+                float *inverse[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    acc[i] = vector(published + (i0 + i) * kSmallPitch + c);
+                    inverse[i] = inverse_row(K, i0 + i);
+                }
+                for (int k0 = 0; k0 <= (tid < 32 ? 12 : 28); k0 += 4) {
+                    float4 l[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) l[i] = vector(inverse[i] + k0);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float4 v = vector(published + (k0 + e) * kSmallPitch + c);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float entry = e == 0 ? l[i].x : (e == 1 ? l[i].y : (e == 2 ? l[i].z : l[i].w));
+                            const float f = k0 + e < i0 + i ? entry : 0.0f;
+                            acc[i].x = fmaf(f, v.x, acc[i].x), acc[i].y = fmaf(f, v.y, acc[i].y);
+                            acc[i].z = fmaf(f, v.z, acc[i].z), acc[i].w = fmaf(f, v.w, acc[i].w);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) vector(u_block + (i0 + i) * kSmallPitch + c) = acc[i];
+            }
+        };
+        // The columns of a block, R rows per thread of `crew` warps: w[h][0] is the next column, and the registers move
+        // down by one as it is eliminated (zeros come in at the top, so a row's registers beyond its
+        // columns are zeros). `home(h, column, entry)` takes the column's own entry, a multiplier or an
+        // entry of U. To keep the chain short
+        //  - only the pivot's row is published (a 16-byte store takes shared memory about six cycles however few
+        //    lanes store: eight warps' candidate rows took 385), and two rows per thread halve the readers;
+        //  - nothing but the loop branches (10 to 20 cycles each): selects and predicated stores, and the number
+        //    of 16-byte pieces a row still has is a constant for eight columns at a time. With branches a column
+        //    took 1030 cycles at order 128; all 32 columns unrolled took 840, waiting for instructions.
+        auto columns_of = [&](auto rows_c, auto &w, auto &line, auto &spot, int crew, int j0, int bw, auto home) {
+            constexpr int R = decltype(rows_c)::value, kCrew = kWarps / R;
+            auto meet = [&] { asm volatile("bar.sync 1, %0;" ::"r"(32 * crew) : "memory"); };
+            static_for<4>([&](auto segment_c) {
+                constexpr int segment = decltype(segment_c)::value, V = 8 - 2 * segment;
+#pragma unroll 1
+                for (int j = 8 * segment; j < (bw < 8 * segment + 8 ? bw : 8 * segment + 8); ++j) {
+                    const int column = j0 + j;
+                    unsigned key[R];
+                    bool live[R];
+#pragma unroll
+                    for (int h = 0; h < R; ++h) {
+                        live[h] = line[h] < n && spot[h] >= column;
+                        const unsigned bits = __float_as_uint(w[h][0]) & 0x7fffffffu;
+                        // |value| + 1; a NaN only stands at the pivot position, where every comparison fails
+                        const unsigned ordinary = bits <= 0x7f800000u ? bits + 1u : (spot[h] == column ? ~0u : 0u);
+                        key[h] = live[h] ? ordinary : 0u;
+                    }
+                    const bool second = R > 1 && (key[R - 1] > key[0] || (key[R - 1] == key[0] && spot[R - 1] < spot[0]));
+                    const unsigned own_key = second ? key[R - 1] : key[0];
+                    const unsigned own_place = static_cast<unsigned>(second ? spot[R - 1] : spot[0]);
+                    const float own_value = second ? w[R - 1][0] : w[0][0];
+                    const unsigned most = __reduce_max_sync(kAll, own_key);
+                    // 1 / value, of use if this row is the pivot's, by one step of Newton's iteration on the approximate
+                    // reciprocal; `scale` keeps that in range
+                    const float size = fabsf(own_value);
+                    const float scale = size < 0x1p-96f ? 0x1p96f : (size > 0x1p96f ? 0x1p-96f : 1.0f);
+                    const float scaled = own_value * scale, guess = __fdividef(1.0f, scaled);
+                    const float reciprocal = fmaf(guess, fmaf(-scaled, guess, 1.0f), guess);
+                    unsigned mine = __ballot_sync(kAll, own_key == most);
+                    if (mine & (mine - 1)) {  // equals: the lowest place
+                        const unsigned lowest = __reduce_min_sync(kAll, own_key == most ? own_place : ~0u);
+                        mine = __ballot_sync(kAll, own_key == most && own_place == lowest);
+                    }
+                    const bool leads = lane == __ffs(mine) - 1;
+                    small_store_if(leads, &best[warp], most, own_place);
+                    meet();
+                    uint2 top = best[0];
+                    int from = 0;
+#pragma unroll
+                    for (int v = 1; v < kCrew; ++v) {
+                        const uint2 other = best[v];
+                        const bool better = other.x > top.x || (other.x == top.x && other.y < top.y);
+                        top.x = better ? other.x : top.x, top.y = better ? other.y : top.y, from = better ? v : from;
+                    }
+                    const bool winner = leads && warp == from;
+                    float *pivot = pivot_rows[j & 1];
+#pragma unroll
+                    for (int h = 0; h < R; ++h) {
+                        const bool publishes = winner && second == (h > 0);
+#pragma unroll
+                        for (int v = 0; v < V; ++v) small_store_if(publishes, pivot + 4 * v, w[h][4 * v], w[h][4 * v + 1], w[h][4 * v + 2], w[h][4 * v + 3]);
+                    }
+                    small_store_if(winner, &pivot_reciprocals[j & 1], __float_as_uint(scale), __float_as_uint(reciprocal));
+                    meet();
+                    float4 u[V + 1];
+                    u[V] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    const float2 inverse = pivot_reciprocals[j & 1];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) u[v] = vector(pivot + 4 * v);
+#pragma unroll
+                    for (int h = 0; h < R; ++h) {
+                        const bool chosen = winner && second == (h > 0);
+                        const bool act = live[h] && !chosen && u[0].x != 0.0f;
+                        const float quotient = w[h][0] * inverse.x * inverse.y;
+                        const float l = act ? quotient : 0.0f;  // a row that is done multiplies by zero
+                        home(h, column, act ? quotient : w[h][0]);
+                        spot[h] = chosen ? column : (spot[h] == column ? static_cast<int>(top.y) : spot[h]);
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            w[h][4 * v] = fmaf(-l, u[v].y, w[h][4 * v + 1]);
+                            w[h][4 * v + 1] = fmaf(-l, u[v].z, w[h][4 * v + 2]);
+                            w[h][4 * v + 2] = fmaf(-l, u[v].w, w[h][4 * v + 3]);
+                            w[h][4 * v + 3] = v < V - 1 ? fmaf(-l, u[v + 1].x, w[h][4 * v + 4 < 32 ? 4 * v + 4 : 0]) : 0.0f;
+                        }
+                    }
+                }
+            });
+        };
+        for (int J = 0; J < nb; ++J) {
+            const int j0 = 32 * J, bw = n - j0 < 32 ? n - j0 : 32;
+            if (RB > 0 && J >= SB) {
+                // a register block: a row per thread
+                float held_rows[1][32], (&w)[32] = held_rows[0];
+#pragma unroll
+                for (int c = 0; c < 32; ++c) w[c] = J == SB ? held[0][c] : held[RB > 1 ? 1 : 0][c];
+                for (int K = 0; K < J; ++K) {
+                    const int q = place - 32 * K;
+                    if (q >= 0 && q < 32) {
+#pragma unroll
+                        for (int c = 0; c < 32; c += 4) vector(published + q * kSmallPitch + c) = make_float4(w[c], w[c + 1], w[c + 2], w[c + 3]);
+                    }
+                    __syncthreads();
+                    product(K);
+                    __syncthreads();
+                    auto subtract_row = [&](int k, float l) {
+                        const unsigned long long f = small_pair(-l, -l);
+#pragma unroll
+                        for (int c = 0; c < 32; c += 4) {
+                            const float4 u = vector(u_block + k * kSmallPitch + c);
+                            small_fma_pair(w[c], w[c + 1], f, u.x, u.y);
+                            small_fma_pair(w[c + 2], w[c + 3], f, u.z, u.w);
+                        }
+                    };
+                    if (q >= 0 && q < 32) {
+#pragma unroll
+                        for (int c = 0; c < 32; c += 4) {
+                            const float4 u = vector(u_block + q * kSmallPitch + c);
+                            w[c] = u.x, w[c + 1] = u.y, w[c + 2] = u.z, w[c + 3] = u.w;
+                        }
+                    } else if (row && q >= 32) {
+                        if (K >= SB) {
+#pragma unroll
+                            for (int k = 0; k < 32; ++k) subtract_row(k, held[0][k]);  // only the first register block precedes another
+                        } else {
+#pragma unroll 1
+                            for (int k = 0; k < 32; k += 4) {
+                                const float4 l = vector(own + 32 * K + k);
+                                subtract_row(k, l.x), subtract_row(k + 1, l.y), subtract_row(k + 2, l.z), subtract_row(k + 3, l.w);
+                            }
+                        }
+                    }
+                }
+                float kept[32];
+                const int line[1] = {tid};
+                int spot[1] = {place};
+                columns_of(Int<1>{}, held_rows, line, spot, warps, j0, bw, [&](int, int, float entry) {
+#pragma unroll
+                    for (int c = 0; c < 31; ++c) kept[c] = kept[c + 1];
+                    kept[31] = entry;
+                });
+                place = spot[0];
+                if (row && place >= j0 && place < j0 + bw) rows[place] = static_cast<unsigned short>(tid);
+#pragma unroll 1
+                for (int j = bw; j < 32; ++j) {
+#pragma unroll
+                    for (int c = 0; c < 31; ++c) kept[c] = kept[c + 1];
+                    kept[31] = 0.0f;
+                }
+#pragma unroll
+                for (int c = 0; c < 32; ++c) {
+                    if (J == SB) held[0][c] = kept[c];
+                    else held[RB > 1 ? 1 : 0][c] = kept[c];
+                }
+                if (row && place >= j0 && place < j0 + bw) {
+#pragma unroll
+                    for (int c = 0; c < 32; c += 4)
+                        vector(u_block + (place - j0) * kSmallPitch + c) = make_float4(kept[c], kept[c + 1], kept[c + 2], kept[c + 3]);
+                }
+            } else {
+                if (J > 0) {
+                    // tiles of 4 rows (eight apart) x 8 columns per lane
+                    const int first = 32 * warp + (lane >> 2), c0 = (lane & 3) * 8;
+                    float t[4][8];
+                    int at[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int line = first + 8 * i;
+                        at[i] = line < n ? places[line] : -1;
+#pragma unroll
+                        for (int h = 0; h < 8; h += 4) {
+                            const float4 v = line < n && j0 + c0 + h < columns ? vector(A + line * P + j0 + c0 + h)
+                                                                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            t[i][h] = v.x, t[i][h + 1] = v.y, t[i][h + 2] = v.z, t[i][h + 3] = v.w;
+                        }
+                    }
+                    for (int K = 0; K < J; ++K) {
+                        bool below = false;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int q = at[i] - 32 * K;
+                            below = below || q >= 32;
+                            if (q >= 0 && q < 32) {
+#pragma unroll
+                                for (int h = 0; h < 8; h += 4)
+                                    vector(published + q * kSmallPitch + c0 + h) = make_float4(t[i][h], t[i][h + 1], t[i][h + 2], t[i][h + 3]);
+                            }
+                        }
+                        __syncthreads();
+                        product(K);
+                        __syncthreads();
+                        if (__any_sync(kAll, below)) {
+#pragma unroll 2
+                            for (int k0 = 0; k0 < 32; k0 += 4) {
+                                float l[4][4];
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const bool live = at[i] >= 32 * K + 32;  // rows placed in or above the block keep theirs
+                                    const float4 v = live ? vector(A + (first + 8 * i) * P + 32 * K + k0)
+                                                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                                    l[i][0] = -v.x, l[i][1] = -v.y, l[i][2] = -v.z, l[i][3] = -v.w;
+                                }
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const float4 u = vector(u_block + (k0 + e) * kSmallPitch + c0);
+                                    const float4 v = vector(u_block + (k0 + e) * kSmallPitch + c0 + 4);
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        const unsigned long long f = small_pair(l[i][e], l[i][e]);
+                                        small_fma_pair(t[i][0], t[i][1], f, u.x, u.y);
+                                        small_fma_pair(t[i][2], t[i][3], f, u.z, u.w);
+                                        small_fma_pair(t[i][4], t[i][5], f, v.x, v.y);
+                                        small_fma_pair(t[i][6], t[i][7], f, v.z, v.w);
+                                    }
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int q = at[i] - 32 * K;
+                            if (q >= 0 && q < 32) {
+#pragma unroll
+                                for (int h = 0; h < 8; h += 4) {
+                                    const float4 u = vector(u_block + q * kSmallPitch + c0 + h);
+                                    t[i][h] = u.x, t[i][h + 1] = u.y, t[i][h + 2] = u.z, t[i][h + 3] = u.w;
+                                }
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int h = 0; h < 8; h += 4)
+                            if (first + 8 * i < n && j0 + c0 + h < columns)
+                                vector(A + (first + 8 * i) * P + j0 + c0 + h) = make_float4(t[i][h], t[i][h + 1], t[i][h + 2], t[i][h + 3]);
+                    __syncthreads();
+                }
+                const int crew = (n + 63) / 64;
+                if (warp < crew) {
+                    float w[2][32];
+                    int line[2], spot[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        line[h] = 64 * warp + 32 * h + lane;
+                        spot[h] = line[h] < n ? places[line[h]] : kSmallMax;
+#pragma unroll
+                        for (int c = 0; c < 32; c += 4) {
+                            const float4 v = line[h] < n && j0 + c < columns ? vector(A + line[h] * P + j0 + c)
+                                                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            w[h][c] = v.x, w[h][c + 1] = v.y, w[h][c + 2] = v.z, w[h][c + 3] = v.w;
+                        }
+                    }
+                    columns_of(Int<2>{}, w, line, spot, crew, j0, bw, [&](int h, int column, float entry) {
+                        if (line[h] < n) A[line[h] * P + column] = entry;
+                    });
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if (line[h] < n) {
+                            places[line[h]] = static_cast<unsigned short>(spot[h]);
+                            if (spot[h] >= j0 && spot[h] < j0 + bw) rows[spot[h]] = static_cast<unsigned short>(line[h]);
+                        }
+                }
+                __syncthreads();
+                if (row) place = places[tid];
+                // the block's L and U (bordered by the identity), for the warps that invert them
+                for (int piece = tid; piece < 8 * bw; piece += blockDim.x) {
+                    const int i = piece >> 3, c = (piece & 7) * 4;
+                    vector(u_block + i * kSmallPitch + c) = j0 + c < columns ? vector(A + rows[j0 + i] * P + j0 + c)
+                                                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+            }
+            for (int i = bw + warp; i < 32; i += warps) u_block[i * kSmallPitch + lane] = lane == i ? 1.0f : 0.0f;
+            __syncthreads();
+            // Both inverses in place, a warp each: the two 16 x 16 diagonal blocks side by side (a lane per column), then the
+            // block between them from the products -X22 (L21 X11) and -Y11 (U12 Y22).
+            auto corner = [&](bool lower) {
+                const int r0 = (lane >> 3) * 4, c0 = (lane & 7) * 2;  // four rows and two columns of the 16 x 16 products
+                float *scratch = published + (lower ? 0 : 16) * kSmallPitch;
+#pragma unroll 1
+                for (int step = 0; step < 2; ++step) {
+                    // first: the off-diagonal block times the inverse of its column's diagonal block; then the inverse of its
+                    // row's diagonal block times that
+                    const bool off = step == 0;
+                    const float *left = off ? (lower ? u_block + 16 * kSmallPitch : u_block + 16)
+                                            : (lower ? u_block + 16 * kSmallPitch + 16 : u_block);
+                    const float *right = off ? (lower ? u_block : u_block + 16 * kSmallPitch + 16) : scratch;
+                    float acc[4][2] = {};
+#pragma unroll
+                    for (int k0 = 0; k0 < 16; k0 += 4) {
+                        float b[4][2];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int k = k0 + e;
+                            const float2 v = *reinterpret_cast<const float2 *>(right + k * kSmallPitch + c0);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const float entry = h == 0 ? v.x : v.y;
+                                const int c = c0 + h;
+                                b[e][h] = !off ? entry : (lower ? (k > c ? entry : (k == c ? 1.0f : 0.0f)) : (k <= c ? entry : 0.0f));
+                            }
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 v = *reinterpret_cast<const float4 *>(left + (r0 + i) * kSmallPitch + k0);
+                            const float line[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int k = k0 + e, at = r0 + i;
+                                const float l = off ? line[e] : (lower ? (k < at ? line[e] : (k == at ? 1.0f : 0.0f)) : (k >= at ? line[e] : 0.0f));
+                                acc[i][0] = fmaf(l, b[e][0], acc[i][0]);
+                                acc[i][1] = fmaf(l, b[e][1], acc[i][1]);
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    float *out = off ? scratch : (lower ? u_block + 16 * kSmallPitch : u_block + 16);
+                    const float sign = off ? 1.0f : -1.0f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        *reinterpret_cast<float2 *>(out + (r0 + i) * kSmallPitch + c0) = make_float2(sign * acc[i][0], sign * acc[i][1]);
+                    __syncwarp();
+                }
+            };
+            const int side = lane & 16, at = lane & 15;  // this lane's diagonal block, and its column of it
+            float *diagonal = u_block + side * kSmallPitch + side;
+            if (warp == 0) {
+                float v[16];
+                static_for<16>([&](auto i_c) {
+                    constexpr int i = decltype(i_c)::value;
+                    float s[4] = {at == i ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int k = 0; k < i; k += 4) {
+                        const float4 l = vector(diagonal + i * kSmallPitch + k);
+                        s[0] = fmaf(-l.x, v[k], s[0]);
+                        if (k + 1 < i) s[1] = fmaf(-l.y, v[k + 1], s[1]);
+                        if (k + 2 < i) s[2] = fmaf(-l.z, v[k + 2], s[2]);
+                        if (k + 3 < i) s[3] = fmaf(-l.w, v[k + 3], s[3]);
+                    }
+                    v[i] = (s[0] + s[1]) + (s[2] + s[3]);
+                });
+                __syncwarp();
+#pragma unroll
+                for (int i = 1; i < 16; ++i)
+                    if (at < i) diagonal[i * kSmallPitch + at] = v[i];
+                __syncwarp();
+                corner(true);
+            }
+            if (warp == (warps > 1 ? 1 : 0)) {
+                float v[16];
+                const float reciprocal = div(1.0f, u_block[lane * kSmallPitch + lane]);
+                static_for<16>([&](auto i_c) {
+                    constexpr int i = 15 - decltype(i_c)::value;
+                    float s[4] = {at == i ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int k = i / 4 * 4; k < 16; k += 4) {
+                        const float4 u = vector(diagonal + i * kSmallPitch + k);
+                        if (k > i) s[0] = fmaf(-u.x, v[k], s[0]);
+                        if (k + 1 > i) s[1] = fmaf(-u.y, v[k + 1], s[1]);
+                        if (k + 2 > i) s[2] = fmaf(-u.z, v[k + 2], s[2]);
+                        if (k + 3 > i) s[3] = fmaf(-u.w, v[k + 3], s[3]);
+                    }
+                    v[i] = ((s[0] + s[1]) + (s[2] + s[3])) * __shfl_sync(kAll, reciprocal, side + i);
+                });
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    if (at >= i) diagonal[i * kSmallPitch + at] = v[i];
+                __syncwarp();
+                corner(false);
+            }
+            __syncthreads();
+            // home: over the block's own rows
+            for (int piece = tid; piece < 8 * bw; piece += blockDim.x) {
+                const int i = piece >> 3, c = (piece & 7) * 4;
+                if ((RB > 0 && J >= SB) || j0 + c < columns) vector(inverse_row(J, i) + c) = vector(u_block + i * kSmallPitch + c);
+            }
+        }
+        __syncthreads();
+
+        // ---- refinement
+        double berr = INFINITY, previous = INFINITY;
+        int count = 0;
+        float c[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) c[q] = static_cast<float>(rhs[q]);
+        // this row's entries of block K, read ahead of the values they multiply
+        auto entries = [&](int K, float (&l)[32]) {
+            if (RB > 0 && K >= SB) {
+#pragma unroll
+                for (int k = 0; k < 32; ++k) l[k] = K == SB ? held[0][k] : held[RB > 1 ? 1 : 0][k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 32; k += 4) {
+                    const float4 v = 32 * K + k < columns ? vector(own + 32 * K + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    l[k] = v.x, l[k + 1] = v.y, l[k + 2] = v.z, l[k + 3] = v.w;
+                }
+            }
+        };
+        auto subtract = [&](const float (&l)[32]) {
+            if constexpr (NR == 1) {
+                float s[2] = {0.0f, 0.0f};
+#pragma unroll
+                for (int k = 0; k < 32; k += 4) {
+                    const float4 v = vector(solved + k);
+                    s[0] = fmaf(l[k], v.x, s[0]), s[1] = fmaf(l[k + 1], v.y, s[1]);
+                    s[0] = fmaf(l[k + 2], v.z, s[0]), s[1] = fmaf(l[k + 3], v.w, s[1]);
+                }
+                c[0] -= s[0] + s[1];
+            } else {
+                static_assert(NR == 1 || NR == 4, "right-hand sides in 16-byte pieces");
+#pragma unroll
+                for (int k = 0; k < 32; ++k) {
+                    const float4 v = vector(solved + k * NR);
+                    c[0] = fmaf(-l[k], v.x, c[0]), c[1 % NR] = fmaf(-l[k], v.y, c[1 % NR]);
+                    c[2 % NR] = fmaf(-l[k], v.z, c[2 % NR]), c[3 % NR] = fmaf(-l[k], v.w, c[3 % NR]);
+                }
+            }
+        };
+        // the product of lane's row of block K's inverse (its entries before `lane` for L, from it on for U) with the block's
+        // right-hand sides; zeros for lanes beyond the block
+        auto solve_block = [&](int K, int bw, bool lower, float (&y)[NR]) {
+            const float *inverse = inverse_row(K, lane < bw ? lane : 0);
+            float s[2][NR];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) s[0][q] = lower ? to_solve[lane * NR + q] : 0.0f, s[1][q] = 0.0f;
+            // all loads first; what lies beyond the block's columns is another row's (or nothing's) and is dropped
+            float4 line[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) line[k] = *reinterpret_cast<const float4 *>(inverse + 4 * k);
+#pragma unroll
+            for (int k0 = 0; k0 < 32; k0 += 4) {
+                const float l[4] = {line[k0 / 4].x, line[k0 / 4].y, line[k0 / 4].z, line[k0 / 4].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int k = k0 + e;
+                    const float f = (lower ? k < lane : (k >= lane && k < bw)) ? l[e] : 0.0f;
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) s[e & 1][q] = fmaf(f, to_solve[k * NR + q], s[e & 1][q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NR; ++q) y[q] = lane < bw ? s[0][q] + s[1][q] : 0.0f;
+        };
+        while (true) {
+#pragma unroll 1
+            for (int K = 0; K < nb; ++K) {
+                const int at = place - 32 * K, bw = n - 32 * K < 32 ? n - 32 * K : 32;
+                const bool below = row && at >= 32;
+                float l[32];
+                if (at >= 0 && at < 32) {
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) to_solve[at * NR + q] = c[q];
+                }
+                __syncthreads();
+                if (below) entries(K, l);
+                if (warp == 0) {
+                    float y[NR];
+                    solve_block(K, bw, true, y);
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) solved[lane * NR + q] = y[q];
+                }
+                __syncthreads();
+                if (at >= 0 && at < 32) {
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) c[q] = solved[at * NR + q];
+                } else if (below) {
+                    subtract(l);
+                }
+            }
+#pragma unroll 1
+            for (int K = nb - 1; K >= 0; --K) {
+                const int at = place - 32 * K, bw = n - 32 * K < 32 ? n - 32 * K : 32;
+                float l[32];
+                if (at >= 0 && at < 32) {
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) to_solve[at * NR + q] = c[q];
+                }
+                __syncthreads();
+                if (at < 0) entries(K, l);  // the rows placed above the block
+                if (warp == 0) {
+                    float y[NR];
+                    solve_block(K, bw, false, y);
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) {
+                        solved[lane * NR + q] = y[q];
+                        if (lane < bw) x[(32 * K + lane) * NR + q] += static_cast<double>(y[q]);
+                    }
+                }
+                __syncthreads();
+                if (at < 0) subtract(l);
+            }
+            // r = b - A x in FP64, with |r_q|_inf and |x_q|_inf
+            double r_max[NR], x_max[NR];
+#pragma unroll
+            for (int q = 0; q < NR; ++q) r_max[q] = 0.0;
+            if (sys.transposed) {
+                if (row) {
+                    double s[NR][2];
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) s[q][0] = s[q][1] = 0.0;
+#pragma unroll 8
+                    for (int k = 0; k + 1 < n; k += 2) {
+                        const double v0 = a[1ll * k * n + tid], v1 = a[1ll * (k + 1) * n + tid];
+#pragma unroll
+                        for (int q = 0; q < NR; ++q) {
+                            s[q][0] = fma(v0, x[k * NR + q], s[q][0]);
+                            s[q][1] = fma(v1, x[(k + 1) * NR + q], s[q][1]);
+                        }
+                    }
+                    if (n & 1) {
+                        const double v = a[1ll * (n - 1) * n + tid];
+#pragma unroll
+                        for (int q = 0; q < NR; ++q) s[q][0] = fma(v, x[(n - 1) * NR + q], s[q][0]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) {
+                        const double residual = rhs[q] - (s[q][0] + s[q][1]);
+                        r[tid * NR + q] = residual;
+                        r_max[q] = fabs(residual);
+                    }
+                }
+            } else {
+                // a warp per row, several rows' loads in flight (as the load); R rows' sums of every right-hand side
+                auto residual = [&](auto g_c) {
+                    constexpr int G = decltype(g_c)::value, R = NR == 1 ? (G <= 4 ? 8 : 4) : 2, M = R * NR;
+                    double v[R][G];
+                    auto fetch = [&](int row0) {
+#pragma unroll
+                        for (int u = 0; u < R; ++u)
+#pragma unroll
+                            for (int g = 0; g < G; ++g) {
+                                const int at = row0 + u * warps, col = lane + 32 * g;
+                                v[u][g] = at < n && col < n ? a[1ll * at * n + col] : 0.0;
+                            }
+                    };
+                    fetch(warp);
+                    for (int row0 = warp; row0 < n; row0 += R * warps) {
+                        double s[M];
+#pragma unroll
+                        for (int m = 0; m < M; ++m) s[m] = 0.0;
+#pragma unroll
+                        for (int g = 0; g < G; ++g) {
+                            const int col = lane + 32 * g;
+#pragma unroll
+                            for (int q = 0; q < NR; ++q) {
+                                const double value = col < n ? x[col * NR + q] : 0.0;
+#pragma unroll
+                                for (int u = 0; u < R; ++u) s[u * NR + q] = fma(v[u][g], value, s[u * NR + q]);
+                            }
+                        }
+                        fetch(row0 + R * warps);  // the next rows' loads, in flight during the sums
+                        int which;
+                        const double total = small_warp_sums<M>(s, lane, which);
+                        const int at = row0 + which / NR * warps, q = which % NR;
+                        if (at < n && lane % (32 / M) == 0) {
+                            const double value = q < static_cast<int>(sys.columns) ? sys.b[1ull * at * sys.pitch + q] : 0.0;
+                            const double left = value - total;
+                            r[at * NR + q] = left;
+#pragma unroll
+                            for (int p = 0; p < NR; ++p)
+                                if (p == q) r_max[p] = small_larger(fabs(left), r_max[p]);
+                        }
+                    }
+                };
+                if (nb == 1) residual(Int<1>{});
+                else if (nb == 2) residual(Int<2>{});
+                else if (nb <= 4) residual(Int<4>{});
+                else residual(Int<8>{});
+            }
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                x_max[q] = row ? fabs(x[tid * NR + q]) : 0.0;
+#pragma unroll
+                for (int offset = 16; offset > 0; offset >>= 1) {
+                    x_max[q] = small_larger(__shfl_xor_sync(kAll, x_max[q], offset), x_max[q]);
+                    r_max[q] = small_larger(__shfl_xor_sync(kAll, r_max[q], offset), r_max[q]);
+                }
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int q = 0; q < NR; ++q) maxima[warp][q] = r_max[q], maxima[warp][NR + q] = x_max[q];
+            }
+            __syncthreads();
+            berr = 0.0;
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                double rm = 0.0, xm = 0.0;
+                for (int v = 0; v < warps; ++v) rm = small_larger(maxima[v][q], rm), xm = small_larger(maxima[v][NR + q], xm);
+                if (q < static_cast<int>(sys.columns)) berr = small_larger(rm / (a_norm * xm + b_norm[q]), berr);
+            }
+            ++count;
+            if (count >= 30 || !(berr > target) || !(berr < 0.5 * previous)) break;
+            previous = berr;
+            if (row) {
+#pragma unroll
+                for (int q = 0; q < NR; ++q) c[q] = static_cast<float>(r[tid * NR + q]);
+            }
+        }
+        if (row) {
+#pragma unroll
+            for (int q = 0; q < NR; ++q)
+                if (q < static_cast<int>(sys.columns)) sys.x[1ull * tid * sys.pitch + q] = x[tid * NR + q];
+        }
+        if (tid == 0) {
+            if (errors) errors[id] = berr;
+            if (iterations) iterations[id] = count;
+        }
+    }
+
+} // namespace sci_cuda

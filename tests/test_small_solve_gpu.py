@@ -1,0 +1,45 @@
+"""Systems of order 256 or less, solved by one CTA each: the edges of its 32-column blocks, of the sizes
+that change its launch or keep columns in registers, and pivoting that moves rows, ties or skips.
+
+The bound is the refinement's own: a normwise backward error of at most 1e-14 (numpy, FP64).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ORDERS = [1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 151, 152, 153, 191, 192, 193, 223, 224, 225, 241, 255, 256]
+
+
+def matrix(kind, n, rng):
+    g = rng.standard_normal((n, n))
+    if kind == "dominant":
+        return g + n * np.eye(n)
+    if kind == "gaussian":
+        return g
+    if kind == "reversed":  # every pivot at the far end
+        return (g * 1e-3 + n * np.eye(n))[::-1].copy()
+    if kind == "ties":  # columns of equal magnitudes
+        return np.where(g > 0, 1.0, -1.0) + 2 * n * np.eye(n)[rng.permutation(n)]
+    return (g + n * np.eye(n)) * 1e-31
+
+
+def backward_error(a, b, x):
+    return np.abs(b - a @ x).max() / (np.abs(a).sum(axis=1).max() * np.abs(x).max() + np.abs(b).max())
+
+
+@pytest.mark.parametrize("kind", ["dominant", "gaussian", "reversed", "ties", "tiny"])
+def test_batched_orders(device, kind):
+    rng = np.random.default_rng(len(kind))
+    a = [matrix(kind, n, rng) for n in ORDERS]
+    b = [rng.standard_normal(n) for n in ORDERS]
+    da, db = [device.array(m.ravel()) for m in a], [device.array(v) for v in b]
+    dx = [device.empty(n, np.float64) for n in ORDERS]
+    errors, iterations = device.empty(len(ORDERS), np.float64), device.empty(len(ORDERS), np.int32)
+    batch = device.solve_batch(ORDERS, [v.pointer for v in da], [v.pointer for v in db], [v.pointer for v in dx], errors,
+                               iterations)
+    batch.launch()
+    for k, n in enumerate(ORDERS):
+        assert backward_error(a[k], b[k], dx[k].numpy()) <= 1e-14, n
+    assert (errors.numpy() <= 1e-14).all() and (iterations.numpy() <= 30).all()
+    batch.close()
