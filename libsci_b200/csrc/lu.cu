@@ -27,6 +27,7 @@
 // most sqrt(n) eps (eps = 2^-53, as LAPACK's DSGESV; at most 1e-14) or stops improving. Only the
 // residual and the update run in FP64.
 #include "context.hpp"
+#include "small_solve.hpp"
 #include "workspace.hpp"
 
 #include <cuda_runtime.h>
@@ -2411,6 +2412,35 @@ namespace sci_cuda {
             }
         }
 
+        // out = -left right^T for tall operands (n x width, width small): 32 x 32 tiles, a thread's four rows share a column
+        // of right. The general product's 128 x 128 tiles leave most SMs idle at these orders (4 tiles, 18 us at order
+        // 200 and width 3).
+        __global__ void __launch_bounds__(256) negative_outer(const double *left, const double *right, double *out, unsigned n,
+                                                              unsigned width) {
+            __shared__ double l[32][33], r[32][33];
+            const unsigned tx = threadIdx.x % 32, ty = threadIdx.x / 32, i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (unsigned k0 = 0; k0 < width; k0 += 32) {
+    #pragma unroll
+                for (unsigned u = 0; u < 4; ++u) {
+                    const unsigned i = ty + 8 * u;
+                    l[i][tx] = i0 + i < n && k0 + tx < width ? left[1ull * (i0 + i) * width + k0 + tx] : 0.0;
+                    r[i][tx] = j0 + i < n && k0 + tx < width ? right[1ull * (j0 + i) * width + k0 + tx] : 0.0;
+                }
+                __syncthreads();
+                const unsigned last = width - k0 < 32 ? width - k0 : 32;
+                for (unsigned k = 0; k < last; ++k) {
+                    const double v = r[tx][k];
+    #pragma unroll
+                    for (unsigned u = 0; u < 4; ++u) acc[u] = fma(l[ty + 8 * u][k], v, acc[u]);
+                }
+                __syncthreads();
+            }
+    #pragma unroll
+            for (unsigned u = 0; u < 4; ++u)
+                if (i0 + ty + 8 * u < n && j0 + tx < n) out[1ull * (i0 + ty + 8 * u) * n + j0 + tx] = 0.0 - acc[u];
+        }
+
         template <typename T> __global__ void transpose_square(const T *in, T *out, unsigned long long n) {
             __shared__ T tile[32][33];
             const unsigned long long r0 = blockIdx.y * 32ull, c0 = blockIdx.x * 32ull;
@@ -2579,6 +2609,9 @@ namespace {
         cudaMemcpyAsync(host + width, a_norm_device, 8, cudaMemcpyDeviceToHost, ctx.stream);
     }
 
+    // The target of refine_loop's stopping test.
+    double refinement_target(unsigned long long n) { return std::min(std::sqrt(static_cast<double>(n)) * 0x1p-53, 1e-14); }
+
     // The refinement loop for a x = b (a n x n, b and x n x width, double): x = 0, r = b; repeat
     // { x += correct(r); r = b - a x in FP64 } until the normwise backward error
     // max_j |r_j|_inf / (|A|_inf |x_j|_inf + |b_j|_inf) is at most sqrt(n) eps (eps = 2^-53, the
@@ -2600,7 +2633,7 @@ namespace {
         }
         const double *b_norm = host, *a_norm = host + width;
         cudaMemsetAsync(x, 0, n * width * 8, ctx.stream);
-        const double target = std::min(std::sqrt(static_cast<double>(n)) * 0x1p-53, 1e-14);
+        const double target = refinement_target(n);
         constexpr int kMaxIterations = 30;
         double previous = INFINITY;
         berr = INFINITY;
@@ -2620,6 +2653,43 @@ namespace {
         return SCI_CUDA_OK;
     }
 
+    // Solves of order kSmallOrder or less: one launch, a CTA per group of right-hand sides (small_solve.cuh), where the
+    // blocked path below takes 40 to 100 launches. The groups factor the matrix each for themselves, on SMs that would
+    // be idle; with more groups than two waves of them the blocked path's single factorisation is the cheaper one.
+    bool small_solve_fits(Context &ctx, unsigned long long n, unsigned long long width, bool transposed) {
+        return n <= kSmallOrder && width <= 2ull * kSmallGroup * ctx.sms &&
+               small_solve_blocks(width, transposed) <= 2u * static_cast<unsigned>(ctx.sms);
+    }
+
+    // Waits for a small solve and takes the largest backward error and iteration count of CTAs [first, last).
+    struct SmallReports {
+        double *errors;
+        int *iterations;
+        unsigned blocks;
+        static unsigned long long bytes(unsigned blocks) { return 12ull * blocks + 16; }
+        int read(Context &ctx) {
+            host = pinned_doubles(ctx, (bytes(blocks) + 7) / 8);
+            if (host == nullptr) return ctx.fail(SCI_CUDA_ERROR_MEMORY, "pinned host memory for the report");
+            if (int code = ctx.check(cudaMemcpyAsync(host, errors, 12ull * blocks, cudaMemcpyDeviceToHost, ctx.stream),
+                                     "reading the small solve's report"))
+                return code;
+            return ctx.drain();
+        }
+        void largest(unsigned first, unsigned last, double &error, int &count) const {
+            const int *counts = reinterpret_cast<const int *>(host + blocks);
+            for (unsigned b = first; b < last; ++b) {
+                error = (host[b] > error || host[b] != host[b]) ? host[b] : error;
+                count = std::max(count, counts[b]);
+            }
+        }
+        double *host{nullptr};
+    };
+
+    bool overlap(const void *p, unsigned long long p_bytes, const void *q, unsigned long long q_bytes) {
+        const auto a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+        return p != nullptr && q != nullptr && a < b + q_bytes && b < a + p_bytes;
+    }
+
 } // namespace
 
 extern "C" int sci_cuda_solve(sci_cuda_context *context, uint32_t precision, uint32_t refine, const void *matrix,
@@ -2637,6 +2707,20 @@ extern "C" int sci_cuda_solve(sci_cuda_context *context, uint32_t precision, uin
                                                  static_cast<unsigned long long>(order), kPanelRows);
     cudaSetDevice(context->device);
     const unsigned long long n = order, nw = order * width;
+    if (refine == SCI_REFINE_FP64 && small_solve_fits(*context, n, width, false)) {
+        const unsigned blocks = small_solve_blocks(width, false);
+        if (int code = context->check(context->solver->reserve(SmallReports::bytes(blocks)), "reserving the solver workspace"))
+            return code;
+        auto *errors = static_cast<double *>(context->solver->memory);
+        SmallReports reports{errors, reinterpret_cast<int *>(errors + blocks), blocks};
+        if (int code = small_solve_call(*context, static_cast<const double *>(matrix), static_cast<const double *>(right),
+                                        static_cast<double *>(solution), nullptr, nullptr, n, width, refinement_target(n),
+                                        reports.errors, reports.iterations))
+            return code;
+        if (int code = reports.read(*context)) return code;
+        if (report) reports.largest(0, blocks, report->backward_error, report->iterations);
+        return SCI_CUDA_OK;
+    }
     const bool wide = precision == SCI_PRECISION_WIDE;
     const size_t element = (wide && refine == SCI_REFINE_NONE) ? 8 : 4;
     const unsigned long long need = n * n * element + n * 8 + kMovements * sizeof(Movement) + n * 4 + nw * 12 + n * 8 + width * 16 +
@@ -2806,6 +2890,40 @@ extern "C" int sci_cuda_solve_gradient(sci_cuda_context *context, uint32_t preci
                                                  static_cast<unsigned long long>(order), kPanelRows);
     cudaSetDevice(context->device);
     const unsigned long long n = order, nw = order * width;
+    // Small systems: both solves in one launch, each with its own factors (A^T's are as quick to make as A's are to reuse, and
+    // the two run side by side). The blocked path writes lambda after it has read the matrix and X's right-hand side, so
+    // lambda may lie over either there; here it may not.
+    if (refine == SCI_REFINE_FP64 && small_solve_fits(*context, n, width, true) &&
+        !overlap(right_gradient, nw * 8, right, nw * 8) && !overlap(right_gradient, nw * 8, matrix, n * n * 8) &&
+        !overlap(right_gradient, nw * 8, solution, nw * 8)) {
+        const unsigned blocks = small_solve_blocks(width, true);
+        const unsigned long long space = (SmallReports::bytes(blocks) + 255) / 256 * 256;
+        if (int code = context->check(context->solver->reserve(space + 2 * (nw * 8 + 256)), "reserving the solver workspace"))
+            return code;
+        auto *errors = static_cast<double *>(context->solver->memory);
+        SmallReports reports{errors, reinterpret_cast<int *>(errors + blocks), blocks};
+        auto *spare = reinterpret_cast<double *>(static_cast<unsigned char *>(context->solver->memory) + space);
+        double *x = solution ? static_cast<double *>(solution) : spare;
+        double *lambda = right_gradient ? static_cast<double *>(right_gradient) : spare + nw;
+        if (int code = small_solve_call(*context, static_cast<const double *>(matrix), static_cast<const double *>(right), x,
+                                        static_cast<const double *>(upstream), lambda, n, width, refinement_target(n),
+                                        reports.errors, reports.iterations))
+            return code;
+        if (matrix_gradient) {
+            const unsigned tiles = static_cast<unsigned>((n + 31) / 32);
+            negative_outer<<<dim3(tiles, tiles), 256, 0, context->stream>>>(lambda, x, static_cast<double *>(matrix_gradient),
+                                                                            static_cast<unsigned>(n), static_cast<unsigned>(width));
+            if (int code = context->check(cudaGetLastError(), "launching the matrix gradient")) return code;
+        }
+        if (int code = reports.read(*context)) return code;
+        if (report) {
+            int forward = 0, transposed = 0;
+            reports.largest(0, blocks / 2, report->backward_error, forward);
+            reports.largest(blocks / 2, blocks, report->backward_error, transposed);
+            report->iterations = forward + transposed;
+        }
+        return SCI_CUDA_OK;
+    }
     const size_t element = precision == SCI_PRECISION_WIDE ? 8 : 4;
     // everything either form carves, generously: matrices, inverses, right-hand-side blocks, norms
     const unsigned long long need = n * n * (8 + element) + inverse_elements(n) * element + nw * 8 * 10 + n * 32 +
