@@ -16,12 +16,11 @@
 //
 // Kernels: the host merges adjacent axes that every operand reads alike (both broadcast or both
 // full), so most calls reduce to one or two axes (a same-shape or scalar operation to one). When
-// the last merged axis is long, blocks walk (row, piece of the last axis) pairs: the row's offsets
-// are computed once per piece and the piece is read and written contiguously (stride 0 or 1 per
-// operand) -- in 16-byte vectors, two per thread, with the code a template argument, when the axis
-// is a whole number of vectors and the arrays are 16-byte aligned; element by element otherwise.
-// Short last axes map each thread's flat index to every operand's offset. HBM bound: bytes = the output written + each operand read once
-// (a broadcast operand mostly from L2).
+// the last merged axis is 64 elements or more, blocks walk (row, piece of the last axis) pairs: the
+// row's offsets are computed once per piece and the piece is read and written contiguously
+// (stride 0 or 1 per operand) in 16-byte vectors, two per thread. Shorter last axes map each
+// thread's flat index to every operand's offset. HBM bound: bytes = the output written + each
+// operand read once (a broadcast operand mostly from L2).
 #include "context.hpp"
 
 #include <cuda_runtime.h>
@@ -34,7 +33,6 @@ namespace sci_cuda {
     namespace {
 
         constexpr int kMaxAxes = 8;
-        constexpr unsigned kPiece = 1024;
         constexpr int kVectorsPerThread = 2;  // 16-byte vectors per thread per piece (vector form)
 
         template <typename T> struct ApplyLaunch {
@@ -96,111 +94,121 @@ namespace sci_cuda {
             }
         }
 
-        // Rows: (row, piece of the last axis) per block step; the last axis is read with stride 0
-        // or 1 per operand.
-        template <typename T> __global__ void __launch_bounds__(256) apply_rows(const __grid_constant__ ApplyLaunch<T> L) {
+        // Rows in 16-byte vectors, two per thread per piece, whatever the row length and the arrays'
+        // alignment: a row's vectors start at the first element that lies on a 16-byte boundary of
+        // the output, and the few elements before and after them are done one by one. An
+        // operand read along the last axis is loaded as a vector where its row lies on the same
+        // boundary (every operand of the output's shape does, in arrays that are 16-byte aligned),
+        // else by elements, which a warp still reads as whole lines; an operand broadcast
+        // along the last axis is one value per row. The code is a template argument, and so is EVEN: rows of
+        // whole vectors in aligned arrays, whose kernel has no ends to look for. A block steps from
+        // piece to piece by adding, not dividing (the 64-bit division, once per two vectors, was a
+        // fifth of the time of the operations that only write). Bound by HBM; at 5001 x 7003 floats, where
+        // rows that are not whole vectors went element by element, and at 16384 x 16384 (one call, events
+        // around it): where((r, 1), x, y) 202 -> 104 us and 493 -> 468, x - (r, 1) 184 -> 73 and
+        // 400 -> 359, (r, 1) + (1, c) 131 -> 56 and 264 -> 211.
+        template <typename T, int CODE, bool EVEN>
+        __global__ void __launch_bounds__(256) apply_vectors(const __grid_constant__ ApplyLaunch<T> L) {
+            constexpr unsigned V = 16 / sizeof(T), U = kVectorsPerThread;
             const int last = L.rank - 1;
-            const unsigned long long columns = L.extent[last];
-            const unsigned long long chunks = (columns + kPiece - 1) / kPiece;
-            const unsigned long long rows = L.count / columns, pieces = rows * chunks;
-            for (unsigned long long piece = blockIdx.x; piece < pieces; piece += gridDim.x) {
-                const unsigned long long row = piece / chunks, c0 = (piece - row * chunks) * kPiece;
+            const unsigned long long columns = L.extent[last], span = 256ull * V * U;
+            const unsigned long long chunks = (columns + (EVEN ? 0 : V - 1) + span - 1) / span;  // up to V - 1 elements come before the vectors
+            const unsigned long long rows = L.count / columns;
+            const unsigned long long row_step = gridDim.x / chunks, chunk_step = gridDim.x - row_step * chunks;
+            unsigned long long row = blockIdx.x / chunks, chunk = blockIdx.x - row * chunks;
+            for (; row < rows; row += row_step, chunk += chunk_step, row += chunk >= chunks, chunk -= chunk >= chunks ? chunks : 0) {
                 unsigned long long rest = row, base[3] = {0, 0, 0};
                 for (int axis = last - 1; axis >= 0; --axis) {
-                    const unsigned long long coordinate = rest % L.extent[axis];
-                    rest /= L.extent[axis];
+                    const unsigned long long above = axis > 0 ? rest / L.extent[axis] : 0;
+                    const unsigned long long coordinate = rest - above * L.extent[axis];
+                    rest = above;
 #pragma unroll
                     for (int k = 0; k < 3; ++k) base[k] += coordinate * L.stride[k][axis];
                 }
                 T *out = L.output + row * columns;
-                for (unsigned long long c = c0 + threadIdx.x; c < c0 + kPiece && c < columns; c += blockDim.x) {
-                    out[c] = apply_shaped<T>(L.code, operand(L, 0, base[0] + c * L.stride[0][last]),
+                // elements before the first boundary of the output
+                const unsigned offset = static_cast<unsigned>(reinterpret_cast<uintptr_t>(out) / sizeof(T)) % V;
+                const unsigned long long head = EVEN || offset == 0 ? 0 : (V - offset < columns ? V - offset : columns);
+                const unsigned long long vectors = (columns - head) / V;
+                const unsigned long long first = chunk * (256 * U) + threadIdx.x;
+                T v[3][U][V];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const T *from = L.input[k] + base[k];
+                    const bool along = L.stride[k][last] != 0;
+                    const bool whole = EVEN || reinterpret_cast<uintptr_t>(from + head) % 16 == 0;
+                    const T single = (L.input[k] && !along) ? *from : T(0);
+#pragma unroll
+                    for (unsigned u = 0; u < U; ++u) {
+                        const unsigned long long at = first + 256 * u;
+                        if (along && at < vectors) {
+                            if (whole) {
+                                load16(from + head + at * V, v[k][u]);
+                            } else {
+#pragma unroll
+                                for (unsigned e = 0; e < V; ++e) v[k][u][e] = from[head + at * V + e];
+                            }
+                        } else {
+#pragma unroll
+                            for (unsigned e = 0; e < V; ++e) v[k][u][e] = single;
+                        }
+                    }
+                }
+#pragma unroll
+                for (unsigned u = 0; u < U; ++u) {
+                    const unsigned long long at = first + 256 * u;
+                    if (at >= vectors) continue;
+                    T r[V];
+#pragma unroll
+                    for (unsigned e = 0; e < V; ++e) r[e] = apply_shaped<T>(CODE, v[0][u][e], v[1][u][e], v[2][u][e]);
+                    store16(out + head + at * V, r);
+                }
+                if constexpr (EVEN) continue;
+                // the elements before and after the vectors: fewer than 2 V
+                const unsigned long long after = columns - head - vectors * V;
+                if (chunk == 0 && threadIdx.x < head + after) {
+                    const unsigned long long c = threadIdx.x < head ? threadIdx.x : columns - after + (threadIdx.x - head);
+                    out[c] = apply_shaped<T>(CODE, operand(L, 0, base[0] + c * L.stride[0][last]),
                                              operand(L, 1, base[1] + c * L.stride[1][last]),
                                              operand(L, 2, base[2] + c * L.stride[2][last]));
                 }
             }
         }
 
-        // Vectors: the last axis in 16-byte vectors, two per thread per piece. Taken when the last
-        // axis is a whole number of vectors and every array is 16-byte aligned, so each row of the
-        // output and of every operand read along the last axis starts on a vector; an operand
-        // broadcast along the last axis is one value per row. The code is a template argument.
-        template <typename T, int CODE>
-        __global__ void __launch_bounds__(256) apply_vectors(const __grid_constant__ ApplyLaunch<T> L) {
-            constexpr int V = 16 / sizeof(T), U = kVectorsPerThread;
-            const int last = L.rank - 1;
-            const unsigned long long columns = L.extent[last];
-            const unsigned long long span = 1ull * blockDim.x * V * U;
-            const unsigned long long chunks = (columns + span - 1) / span;
-            const unsigned long long pieces = (L.count / columns) * chunks;
-            for (unsigned long long piece = blockIdx.x; piece < pieces; piece += gridDim.x) {
-                const unsigned long long row = piece / chunks, c0 = (piece - row * chunks) * span;
-                unsigned long long rest = row, base[3] = {0, 0, 0};
-                for (int axis = last - 1; axis >= 0; --axis) {
-                    const unsigned long long coordinate = rest % L.extent[axis];
-                    rest /= L.extent[axis];
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) base[k] += coordinate * L.stride[k][axis];
-                }
-                T v[3][U][V];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const bool along = L.stride[k][last] != 0;
-                    const T single = (L.input[k] && !along) ? L.input[k][base[k]] : T(0);
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const unsigned long long c = c0 + (1ull * u * blockDim.x + threadIdx.x) * V;
-                        if (along && c < columns) {
-                            load16(L.input[k] + base[k] + c, v[k][u]);
-                        } else {
-#pragma unroll
-                            for (int e = 0; e < V; ++e) v[k][u][e] = single;
-                        }
-                    }
-                }
-                T *out = L.output + row * columns;
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const unsigned long long c = c0 + (1ull * u * blockDim.x + threadIdx.x) * V;
-                    if (c >= columns) continue;
-                    T r[V];
-#pragma unroll
-                    for (int e = 0; e < V; ++e) r[e] = apply_shaped<T>(CODE, v[0][u][e], v[1][u][e], v[2][u][e]);
-                    store16(out + c, r);
-                }
-            }
-        }
-
-        template <typename T, int CODE> void launch_vectors(Context &ctx, const ApplyLaunch<T> &L) {
+        template <typename T, int CODE, bool EVEN> void launch_vectors(Context &ctx, const ApplyLaunch<T> &L) {
             constexpr int V = 16 / sizeof(T);
             const unsigned long long columns = L.extent[L.rank - 1], span = 256ull * V * kVectorsPerThread;
-            const unsigned long long pieces = (L.count / columns) * ((columns + span - 1) / span);
+            const unsigned long long pieces = (L.count / columns) * ((columns + (EVEN ? 0 : V - 1) + span - 1) / span);
             // one wave: as many blocks as stay resident
             const unsigned long long most =
-                    1ull * ctx.sms * ctx.blocks_per_sm(reinterpret_cast<const void *>(&apply_vectors<T, CODE>), 256, 0);
-            apply_vectors<T, CODE><<<static_cast<unsigned>(pieces < most ? pieces : most), 256, 0, ctx.stream>>>(L);
+                    1ull * ctx.sms * ctx.blocks_per_sm(reinterpret_cast<const void *>(&apply_vectors<T, CODE, EVEN>), 256, 0);
+            apply_vectors<T, CODE, EVEN><<<static_cast<unsigned>(pieces < most ? pieces : most), 256, 0, ctx.stream>>>(L);
+        }
+        template <typename T, int CODE> void launch_vectors(Context &ctx, const ApplyLaunch<T> &L) {
+            auto aligned = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+            if (L.extent[L.rank - 1] % (16 / sizeof(T)) == 0 && aligned(L.output) && aligned(L.input[0]) && aligned(L.input[1]) &&
+                aligned(L.input[2]))
+                launch_vectors<T, CODE, true>(ctx, L);
+            else launch_vectors<T, CODE, false>(ctx, L);
         }
 
-        template <typename T> bool launch_vector_code(Context &ctx, const ApplyLaunch<T> &L) {
+        template <typename T> void launch_vector_code(Context &ctx, const ApplyLaunch<T> &L) {
             switch (L.code) {
-            case SCI_CODE_COPY: launch_vectors<T, SCI_CODE_COPY>(ctx, L); return true;
-            case SCI_CODE_ADD: launch_vectors<T, SCI_CODE_ADD>(ctx, L); return true;
-            case SCI_CODE_SUBTRACT: launch_vectors<T, SCI_CODE_SUBTRACT>(ctx, L); return true;
-            case SCI_CODE_MULTIPLY: launch_vectors<T, SCI_CODE_MULTIPLY>(ctx, L); return true;
-            case SCI_CODE_DIVIDE: launch_vectors<T, SCI_CODE_DIVIDE>(ctx, L); return true;
-            case SCI_CODE_MINIMUM: launch_vectors<T, SCI_CODE_MINIMUM>(ctx, L); return true;
-            case SCI_CODE_MAXIMUM: launch_vectors<T, SCI_CODE_MAXIMUM>(ctx, L); return true;
-            case SCI_EXTRA_FLOOR: launch_vectors<T, SCI_EXTRA_FLOOR>(ctx, L); return true;
-            case SCI_EXTRA_CEIL: launch_vectors<T, SCI_EXTRA_CEIL>(ctx, L); return true;
-            case SCI_EXTRA_ROUND: launch_vectors<T, SCI_EXTRA_ROUND>(ctx, L); return true;
-            case SCI_EXTRA_POWER: launch_vectors<T, SCI_EXTRA_POWER>(ctx, L); return true;
-            case SCI_EXTRA_CLIP: launch_vectors<T, SCI_EXTRA_CLIP>(ctx, L); return true;
-            case SCI_EXTRA_WHERE: launch_vectors<T, SCI_EXTRA_WHERE>(ctx, L); return true;
-            default: return false;
+            case SCI_CODE_COPY: launch_vectors<T, SCI_CODE_COPY>(ctx, L); return;
+            case SCI_CODE_ADD: launch_vectors<T, SCI_CODE_ADD>(ctx, L); return;
+            case SCI_CODE_SUBTRACT: launch_vectors<T, SCI_CODE_SUBTRACT>(ctx, L); return;
+            case SCI_CODE_MULTIPLY: launch_vectors<T, SCI_CODE_MULTIPLY>(ctx, L); return;
+            case SCI_CODE_DIVIDE: launch_vectors<T, SCI_CODE_DIVIDE>(ctx, L); return;
+            case SCI_CODE_MINIMUM: launch_vectors<T, SCI_CODE_MINIMUM>(ctx, L); return;
+            case SCI_CODE_MAXIMUM: launch_vectors<T, SCI_CODE_MAXIMUM>(ctx, L); return;
+            case SCI_EXTRA_FLOOR: launch_vectors<T, SCI_EXTRA_FLOOR>(ctx, L); return;
+            case SCI_EXTRA_CEIL: launch_vectors<T, SCI_EXTRA_CEIL>(ctx, L); return;
+            case SCI_EXTRA_ROUND: launch_vectors<T, SCI_EXTRA_ROUND>(ctx, L); return;
+            case SCI_EXTRA_POWER: launch_vectors<T, SCI_EXTRA_POWER>(ctx, L); return;
+            case SCI_EXTRA_CLIP: launch_vectors<T, SCI_EXTRA_CLIP>(ctx, L); return;
+            default: launch_vectors<T, SCI_EXTRA_WHERE>(ctx, L);
             }
         }
-
-        bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
         int arity(uint32_t code) {
             switch (code) {
@@ -226,16 +234,9 @@ namespace sci_cuda {
             }
             L.output = static_cast<T *>(output);
             L.count = count;
-            const unsigned long long columns = extent[rank - 1];
-            bool vectors = columns % (16 / sizeof(T)) == 0 && aligned16(output);
-            for (int k = 0; k < operands; ++k) vectors = vectors && aligned16(inputs[k]);
-            if (vectors && columns >= 64 && launch_vector_code<T>(ctx, L)) {
-                return ctx.check(cudaGetLastError(), "launching a broadcast operation");
-            }
-            if (columns >= 256) {
-                const unsigned long long pieces = (count / columns) * ((columns + kPiece - 1) / kPiece);
-                const unsigned long long most = 8ull * ctx.sms;
-                apply_rows<T><<<static_cast<unsigned>(pieces < most ? pieces : most), 256, 0, ctx.stream>>>(L);
+            // Rows shorter than 64 elements leave most of a block without a vector: a flat index per element there.
+            if (extent[rank - 1] >= 64) {
+                launch_vector_code<T>(ctx, L);
             } else {
                 const unsigned long long wanted = (count + 255) / 256, most = 8ull * ctx.sms;
                 apply_flat<T><<<static_cast<unsigned>(wanted < most ? wanted : most), 256, 0, ctx.stream>>>(L);
