@@ -12,9 +12,15 @@
 //     (coalesced) and fold with shuffles in a fixed order;
 //   - inner > 1: a thread per (o, piece, j), j fastest, so a warp reads 32 consecutive elements
 //     per k -- or, when inner is a whole number of 16-byte vectors, a thread per (o, piece, vector
-//     of j) reading 512 bytes per warp per k (rows shorter than 64 take the scalar form, a thread
-//     per row);
-// Short outputs over long axes split the axis into pieces so the grid fills the GPU; pieces write
+//     of j) reading 512 bytes per warp per k (rows shorter than 64 take this form, a thread
+//     per row).
+// Each lane keeps 8 to 16 loads in flight ahead of its ordered fold, and the kind of fold is a template
+// argument. Sum over axis 0 and mean over axis 1 of 16384 x 16384 floats (one call, events around
+// it): 233 -> 189 us (5.7 TB/s) and 199 -> 184; of 5001 x 7003: 54 -> 47 and 45 -> 38. A block per 128
+// columns, its warps' folds combined in shared memory, took 370 us for the first (512 bytes of a row
+// at a time instead of 4 KB).
+// Short outputs over long axes split the axis
+// into pieces so the grid fills the GPU; pieces write
 // double partials that one more pass folds in piece order. The order of every fold is fixed by the
 // shape alone, so results are deterministic. HBM bound: the input is read once.
 #include "context.hpp"
@@ -29,6 +35,7 @@ using namespace sci_cuda;
 namespace sci_cuda {
     namespace {
 
+        // `fold` is a constant in the wide forms, so that their inner loops do not choose.
         __device__ __forceinline__ double fold_pair(unsigned fold, double a, double b) {
             if (fold == SCI_FOLD_SUM) return __dadd_rn(a, b);
             if (a != a) return a;
@@ -59,8 +66,9 @@ namespace sci_cuda {
             unsigned folded;  // the fold applied to values (mean folds as a sum)
         };
 
-        template <typename T>
+        template <typename T, unsigned FOLD>
         __global__ void __launch_bounds__(256) axis_rows(const T *in, AxisShape s, double *partial, T *out) {
+            constexpr int U = 16;  // loads in flight per lane
             const unsigned lane = threadIdx.x & 31;
             const unsigned long long warps = 1ull * gridDim.x * (blockDim.x >> 5);
             const unsigned long long units = s.outer * s.pieces;
@@ -68,12 +76,26 @@ namespace sci_cuda {
                 const unsigned long long row = unit / s.pieces, piece = unit - row * s.pieces;
                 const unsigned long long k0 = piece * s.span, k1 = k0 + s.span < s.extent ? k0 + s.span : s.extent;
                 const T *line = in + row * s.extent;
-                double acc = fold_start(s.folded);
-#pragma unroll 4
-                for (unsigned long long k = k0 + lane; k < k1; k += 32) acc = fold_pair(s.folded, acc, static_cast<double>(line[k]));
+                double acc = fold_start(FOLD);
+                unsigned long long k = k0 + lane;
+                for (; k + 32ull * (U - 1) < k1; k += 32ull * U) {
+                    T v[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v[u] = line[k + 32ull * u];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) acc = fold_pair(FOLD, acc, static_cast<double>(v[u]));
+                }
+                // the rest: the same loads, each where there is an element
+                T v[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k + 32ull * u < k1) v[u] = line[k + 32ull * u];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (k + 32ull * u < k1) acc = fold_pair(FOLD, acc, static_cast<double>(v[u]));
 #pragma unroll
                 for (int offset = 16; offset > 0; offset >>= 1)
-                    acc = fold_pair(s.folded, acc, __shfl_xor_sync(0xffffffffu, acc, offset));
+                    acc = fold_pair(FOLD, acc, __shfl_xor_sync(0xffffffffu, acc, offset));
                 if (lane == 0) {
                     if (s.pieces == 1) out[row] = finish<T>(s.fold, acc, s.extent);
                     else partial[unit] = acc;
@@ -81,51 +103,45 @@ namespace sci_cuda {
             }
         }
 
-        template <typename T>
+        // Columns: a thread per (o, piece, group of C adjacent columns), each folding its columns in the order of k. C is a
+        // 16-byte vector's width when inner is a whole number of vectors and the input 16-byte aligned, else 1.
+        template <typename T, unsigned FOLD, int C>
         __global__ void __launch_bounds__(256) axis_columns(const T *in, AxisShape s, double *partial, T *out) {
+            constexpr int U = 16 / C < 8 ? 8 : 16 / C;  // loads in flight
             const unsigned long long threads = 1ull * gridDim.x * blockDim.x;
-            const unsigned long long units = s.outer * s.pieces * s.inner;
-            for (unsigned long long unit = 1ull * blockIdx.x * blockDim.x + threadIdx.x; unit < units; unit += threads) {
-                const unsigned long long j = unit % s.inner, rest = unit / s.inner;
-                const unsigned long long piece = rest % s.pieces, o = rest / s.pieces;
-                const unsigned long long k0 = piece * s.span, k1 = k0 + s.span < s.extent ? k0 + s.span : s.extent;
-                const T *column = in + o * s.extent * s.inner + j;
-                double acc = fold_start(s.folded);
-                // unrolled so eight loads are in flight ahead of the (ordered) fold
-#pragma unroll 8
-                for (unsigned long long k = k0; k < k1; ++k) acc = fold_pair(s.folded, acc, static_cast<double>(column[k * s.inner]));
-                if (s.pieces == 1) out[o * s.inner + j] = finish<T>(s.fold, acc, s.extent);
-                else partial[unit] = acc;
-            }
-        }
-
-        // The column form over 16-byte vectors of adjacent columns (inner a whole number of vectors,
-        // input 16-byte aligned): a thread per (o, piece, vector of j), each lane folding its own
-        // column in the same order as the scalar form.
-        template <typename T>
-        __global__ void __launch_bounds__(256) axis_column_vectors(const T *in, AxisShape s, double *partial, T *out) {
-            constexpr int V = 16 / sizeof(T);
-            const unsigned long long threads = 1ull * gridDim.x * blockDim.x;
-            const unsigned long long groups = s.inner / V;
+            const unsigned long long groups = s.inner / C;
             const unsigned long long units = s.outer * s.pieces * groups;
             for (unsigned long long unit = 1ull * blockIdx.x * blockDim.x + threadIdx.x; unit < units; unit += threads) {
-                const unsigned long long g = unit % groups, rest = unit / groups;
-                const unsigned long long piece = rest % s.pieces, o = rest / s.pieces;
+                const unsigned long long rest = unit / groups, g = unit - rest * groups;
+                const unsigned long long o = rest / s.pieces, piece = rest - o * s.pieces;
                 const unsigned long long k0 = piece * s.span, k1 = k0 + s.span < s.extent ? k0 + s.span : s.extent;
-                const T *column = in + o * s.extent * s.inner + g * V;
-                double acc[V];
+                const T *column = in + o * s.extent * s.inner + g * C;
+                double acc[C];
 #pragma unroll
-                for (int e = 0; e < V; ++e) acc[e] = fold_start(s.folded);
-#pragma unroll 4
-                for (unsigned long long k = k0; k < k1; ++k) {
-                    T v[V];
-                    load16(column + k * s.inner, v);
+                for (int e = 0; e < C; ++e) acc[e] = fold_start(FOLD);
+                auto read = [&](unsigned long long k, T *v) {
+                    if constexpr (C > 1) load16(column + k * s.inner, v);
+                    else v[0] = column[k * s.inner];
+                };
+                unsigned long long k = k0;
+                for (; k + U <= k1; k += U) {
+                    T v[U][C];
 #pragma unroll
-                    for (int e = 0; e < V; ++e) acc[e] = fold_pair(s.folded, acc[e], static_cast<double>(v[e]));
+                    for (int u = 0; u < U; ++u) read(k + u, v[u]);
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int e = 0; e < C; ++e) acc[e] = fold_pair(FOLD, acc[e], static_cast<double>(v[u][e]));
+                }
+                for (; k < k1; ++k) {
+                    T v[C];
+                    read(k, v);
+#pragma unroll
+                    for (int e = 0; e < C; ++e) acc[e] = fold_pair(FOLD, acc[e], static_cast<double>(v[e]));
                 }
 #pragma unroll
-                for (int e = 0; e < V; ++e) {
-                    const unsigned long long j = g * V + e;
+                for (int e = 0; e < C; ++e) {
+                    const unsigned long long j = g * C + e;
                     if (s.pieces == 1) out[o * s.inner + j] = finish<T>(s.fold, acc[e], s.extent);
                     else partial[(o * s.pieces + piece) * s.inner + j] = acc[e];
                 }
@@ -139,34 +155,38 @@ namespace sci_cuda {
             for (unsigned long long i = 1ull * blockIdx.x * blockDim.x + threadIdx.x; i < outputs; i += step) {
                 const unsigned long long o = i / s.inner, j = i - o * s.inner;
                 double acc = fold_start(s.folded);
+                // eight loads in flight ahead of the (ordered) fold
+#pragma unroll 8
                 for (unsigned long long p = 0; p < s.pieces; ++p) acc = fold_pair(s.folded, acc, partial[(o * s.pieces + p) * s.inner + j]);
                 out[i] = finish<T>(s.fold, acc, s.extent);
             }
         }
 
-        template <typename T> int launch_axis(Context &ctx, const T *in, T *out, AxisShape s) {
-            // Work units for four resident waves of threads, run by one persistent wave, so the last
-            // units do not leave most of the GPU idle.
-            const void *kernel = s.inner == 1 && s.extent >= 64 ? reinterpret_cast<const void *>(&axis_rows<T>)
-                                                                : reinterpret_cast<const void *>(&axis_column_vectors<T>);
-            const unsigned long long most = 1ull * ctx.sms * ctx.blocks_per_sm(kernel, 256, 0);  // blocks of 256
-            const unsigned long long target = 4 * most * 256;                                     // threads' worth of units
-            // short rows go a thread per row (the column form with inner = 1)
-            const bool rows = s.inner == 1 && s.extent >= 64;
-            constexpr unsigned long long V = 16 / sizeof(T);
+        template <typename T, unsigned FOLD> int launch_axis(Context &ctx, const T *in, T *out, AxisShape s) {
+            // Work units for several resident waves, run by one persistent wave, so the last units do not leave most of the
+            // GPU idle.
+            constexpr int V = 16 / sizeof(T);
+            const bool rows = s.inner == 1 && s.extent >= 64;  // shorter rows go a thread per row
             const bool vectors = !rows && s.inner % V == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
+            const void *kernel = rows      ? reinterpret_cast<const void *>(&axis_rows<T, FOLD>)
+                                 : vectors ? reinterpret_cast<const void *>(&axis_columns<T, FOLD, V>)
+                                           : reinterpret_cast<const void *>(&axis_columns<T, FOLD, 1>);
+            const unsigned long long most = 1ull * ctx.sms * ctx.blocks_per_sm(kernel, 256, 0);  // blocks of 256
+            unsigned long long want, cap;
             if (rows) {
-                // a warp per (row, piece); pieces of at least 2048 values
-                const unsigned long long want = (target / 32 + s.outer - 1) / s.outer;
-                const unsigned long long cap = (s.extent + 2047) / 2048;
-                s.pieces = want < cap ? want : cap;
+                // a warp per (row, piece): a wave of warps, in pieces of at least 2048 values
+                want = (8 * most + s.outer - 1) / s.outer;
+                cap = (s.extent + 2047) / 2048;
+                // a row per warp fills two thirds of a wave: no pieces, and no pass to fold them (5001 rows
+                // of 7003 floats: 35 + 4 us in pieces, 33 without)
+                if (s.outer * 3 >= 8 * most * 2) want = 1;
             } else {
-                // a thread per (o, piece, j or vector of j); pieces of at least 64 values
-                const unsigned long long columns = s.outer * (vectors ? s.inner / V : s.inner);
-                const unsigned long long want = (target + columns - 1) / columns;
-                const unsigned long long cap = (s.extent + 63) / 64;
-                s.pieces = want < cap ? want : cap;
+                // a thread per (o, piece, group of columns): four waves, in pieces of at least 64 values
+                const unsigned long long groups = s.outer * (vectors ? s.inner / V : s.inner);
+                want = (4 * most * 256 + groups - 1) / groups;
+                cap = (s.extent + 63) / 64;
             }
+            s.pieces = want < cap ? want : cap;
             if (s.pieces < 1) s.pieces = 1;
             s.span = (s.extent + s.pieces - 1) / s.pieces;
             s.pieces = (s.extent + s.span - 1) / s.span;
@@ -177,24 +197,28 @@ namespace sci_cuda {
                     return code;
                 partial = static_cast<double *>(ctx.workspace->memory);
             }
+            auto grid = [&](unsigned long long blocks) { return static_cast<unsigned>(blocks < most ? blocks : most); };
             if (rows) {
-                const unsigned long long blocks = (s.outer * s.pieces + 7) / 8;
-                axis_rows<T><<<static_cast<unsigned>(blocks < most ? blocks : most), 256, 0, ctx.stream>>>(in, s, partial, out);
+                axis_rows<T, FOLD><<<grid((s.outer * s.pieces + 7) / 8), 256, 0, ctx.stream>>>(in, s, partial, out);
             } else if (vectors) {
-                const unsigned long long blocks = (s.outer * s.pieces * (s.inner / V) + 255) / 256;
-                axis_column_vectors<T><<<static_cast<unsigned>(blocks < most ? blocks : most), 256, 0, ctx.stream>>>(in, s, partial,
-                                                                                                                   out);
+                axis_columns<T, FOLD, V><<<grid((s.outer * s.pieces * (s.inner / V) + 255) / 256), 256, 0, ctx.stream>>>(in, s, partial, out);
             } else {
-                const unsigned long long blocks = (s.outer * s.pieces * s.inner + 255) / 256;
-                axis_columns<T><<<static_cast<unsigned>(blocks < most ? blocks : most), 256, 0, ctx.stream>>>(in, s, partial, out);
+                axis_columns<T, FOLD, 1><<<grid((s.outer * s.pieces * s.inner + 255) / 256), 256, 0, ctx.stream>>>(in, s, partial, out);
             }
             if (int code = ctx.check(cudaGetLastError(), "launching an axis reduction")) return code;
             if (s.pieces > 1) {
-                const unsigned long long blocks = (s.outer * s.inner + 255) / 256;
-                axis_pieces<T><<<static_cast<unsigned>(blocks < most ? blocks : most), 256, 0, ctx.stream>>>(partial, s, out);
+                axis_pieces<T><<<grid((s.outer * s.inner + 255) / 256), 256, 0, ctx.stream>>>(partial, s, out);
                 if (int code = ctx.check(cudaGetLastError(), "launching the axis piece fold")) return code;
             }
             return SCI_CUDA_OK;
+        }
+
+        template <typename T> int launch_fold(Context &ctx, const void *in, void *out, const AxisShape &s) {
+            const T *from = static_cast<const T *>(in);
+            T *to = static_cast<T *>(out);
+            if (s.folded == SCI_FOLD_MINIMUM) return launch_axis<T, SCI_FOLD_MINIMUM>(ctx, from, to, s);
+            if (s.folded == SCI_FOLD_MAXIMUM) return launch_axis<T, SCI_FOLD_MAXIMUM>(ctx, from, to, s);
+            return launch_axis<T, SCI_FOLD_SUM>(ctx, from, to, s);
         }
 
     } // namespace
@@ -227,7 +251,6 @@ extern "C" int sci_cuda_reduce_axis(sci_cuda_context *context, uint32_t precisio
     if (!input || !reachable(*context, input)) return context->fail(SCI_CUDA_ERROR_INVALID, "reduce_axis: the input is not memory of this device");
     if (input == output) return context->fail(SCI_CUDA_ERROR_INVALID, "reduce_axis: the output must not be the input");
     cudaSetDevice(context->device);
-    if (precision == SCI_PRECISION_WIDE)
-        return launch_axis<double>(*context, static_cast<const double *>(input), static_cast<double *>(output), s);
-    return launch_axis<float>(*context, static_cast<const float *>(input), static_cast<float *>(output), s);
+    if (precision == SCI_PRECISION_WIDE) return launch_fold<double>(*context, input, output, s);
+    return launch_fold<float>(*context, input, output, s);
 }
