@@ -576,9 +576,11 @@ namespace sci_cuda {
         unpair(sub(mul(exponent, pair(L::natural)), sub(sub(half, inner), fraction)), r0, r1);
     }
 
-    // circular_fast<phase> on two elements.
-    template <bool phase>
-    __device__ __forceinline__ void circular_pair(float x0, float x1, bool &rare, float &r0, float &r1) {
+    // The reduction, sines and cosines of circular_fast on two elements, before the quadrant picks one.
+    struct CircularPair {
+        float sine[2], cosine[2], shifted[2];
+    };
+    __device__ __forceinline__ CircularPair circular_parts(float x0, float x1, bool &rare) {
         using L = Limits<float>;
         constexpr Poly<float, L::sin_terms> odd = alternating<float, L::sin_terms, 1>();
         constexpr Poly<float, L::cos_terms> even = alternating<float, L::cos_terms, 0>();
@@ -593,22 +595,37 @@ namespace sci_cuda {
         const Pair square = mul(reduced, reduced);
         const Pair sine = fma_(mul(reduced, square), horner<1>(odd, square), reduced);
         const Pair cosine = fma_(square, horner<1>(even, square), pair(1.0f));
-        float s[2], c[2], h[2], out[2];
-        unpair(sine, s[0], s[1]);
-        unpair(cosine, c[0], c[1]);
-        unpair(shifted, h[0], h[1]);
-        // Per lane, q = the low bits of `shifted`: bit 0 swaps sine and cosine, and the sign flips
-        // with bit 1 of q for the sine, with bit 1 of q ^ (q << 1) = bit 1 of q + 1 for the cosine
-        // (the forms above); shifted left by 30 either lands on the sign bit.
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const unsigned q = bits(h[i]);
-            const unsigned sign = ((phase ? q + 1u : q) << 30) & 0x80000000u;
-            const float result = ((q & 1u) != 0) != phase ? c[i] : s[i];
-            out[i] = from_bits(bits(result) ^ sign);
-        }
-        r0 = out[0];
-        r1 = out[1];
+        CircularPair parts;
+        unpair(sine, parts.sine[0], parts.sine[1]);
+        unpair(cosine, parts.cosine[0], parts.cosine[1]);
+        unpair(shifted, parts.shifted[0], parts.shifted[1]);
+        return parts;
+    }
+    // Lane i's sine (phase false) or cosine. q = the low bits of `shifted`: bit 0 swaps sine and cosine, and
+    // the sign flips with bit 1 of q for the sine, with bit 1 of q ^ (q << 1) = bit 1 of q + 1 for the
+    // cosine (the forms above); shifted left by 30 either lands on the sign bit.
+    template <bool phase> __device__ __forceinline__ float circular_pick(const CircularPair &parts, int i) {
+        const unsigned q = bits(parts.shifted[i]);
+        const unsigned sign = ((phase ? q + 1u : q) << 30) & 0x80000000u;
+        const float result = ((q & 1u) != 0) != phase ? parts.cosine[i] : parts.sine[i];
+        return from_bits(bits(result) ^ sign);
+    }
+
+    // circular_fast<phase> on two elements.
+    template <bool phase>
+    __device__ __forceinline__ void circular_pair(float x0, float x1, bool &rare, float &r0, float &r1) {
+        const CircularPair parts = circular_parts(x0, x1, rare);
+        r0 = circular_pick<phase>(parts, 0);
+        r1 = circular_pick<phase>(parts, 1);
+    }
+    // Both at once, `phase` first: the value and the derivative's other half share the reduction.
+    template <bool phase>
+    __device__ __forceinline__ void circular_both(float x0, float x1, bool &rare, float &r0, float &r1, float &o0, float &o1) {
+        const CircularPair parts = circular_parts(x0, x1, rare);
+        r0 = circular_pick<phase>(parts, 0);
+        r1 = circular_pick<phase>(parts, 1);
+        o0 = circular_pick<!phase>(parts, 0);
+        o1 = circular_pick<!phase>(parts, 1);
     }
 
     template <int code, typename T> __device__ __forceinline__ constexpr bool has_pair() {
