@@ -65,8 +65,6 @@ namespace sci_cuda {
             }
         }
 
-        // A (rows x k, pitch lda) into K-major terms, rows x kp: eight values per thread step, read as
-        // two 16-byte vectors where the row allows it.
         // Programmatic dependent launch: returns once the kernel before this one on the stream has
         // finished and its writes are visible, and lets the kernel after this one launch. Both are
         // no-ops in a kernel launched the ordinary way.
@@ -75,68 +73,92 @@ namespace sci_cuda {
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         }
 
-        __global__ void split_rows(const float *__restrict__ a, unsigned long long lda, Terms out, int terms,
-                                   unsigned long long rows, unsigned long long k, unsigned long long kp) {
-            follow_previous();
-            const unsigned long long per_row = kp / 8, total = rows * per_row;
-            const bool vector = lda % 4 == 0 && reinterpret_cast<unsigned long long>(a) % 16 == 0;
-            for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < total; i += 256ull * gridDim.x) {
-                const unsigned long long r = i / per_row, c = (i - r * per_row) * 8;
-                const float *src = a + r * lda + c;
+        // One operand's conversion: `lines` K-major lines of kp values, read from lines of the matrix (pitch ld) or,
+        // transposed, from its columns.
+        struct SplitJob {
+            const float *from;
+            unsigned long long ld, lines, k, kp;
+            Terms out;
+            int transposed;
+            unsigned blocks;
+        };
+
+        // Lines read as they lie: eight values per thread step, two 16-byte vectors where the line allows it.
+        __device__ __forceinline__ void split_lines(const SplitJob &job, int terms, unsigned block) {
+            const unsigned long long per_line = job.kp / 8, total = job.lines * per_line;
+            const bool vector = job.ld % 4 == 0 && reinterpret_cast<unsigned long long>(job.from) % 16 == 0;
+            for (unsigned long long i = block * 256ull + threadIdx.x; i < total; i += 256ull * job.blocks) {
+                const unsigned long long r = i / per_line, c = (i - r * per_line) * 8;
+                const float *src = job.from + r * job.ld + c;
                 float v[8];
-                if (vector && c + 8 <= k) {
+                if (vector && c + 8 <= job.k) {
                     const float4 lo = *reinterpret_cast<const float4 *>(src), hi = *reinterpret_cast<const float4 *>(src + 4);
                     v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = c + e < k ? src[e] : 0.0f;
+                    for (int e = 0; e < 8; ++e) v[e] = c + e < job.k ? src[e] : 0.0f;
                 }
-                split_eight(v, terms, out, r * kp + c);
+                split_eight(v, terms, job.out, r * job.kp + c);
             }
         }
 
-        // B is K x N row-major (pitch ldb); its terms are the transpose, N x Kp, so both operands are
-        // K-major. 64 x 64 tiles through shared memory: read as 16-byte vectors along N, written as
-        // 16-byte vectors (eight K values) along K, eight lanes covering one output row's 64 K values
-        // so each warp's stores are whole 128-byte lines (one lane per row left every 32-byte sector
+        // Columns of a K x N matrix: 64 x 64 tiles through shared memory, read as 16-byte vectors along N, written as
+        // 16-byte vectors (eight K values) along K, eight lanes covering one output line's 64 K values
+        // so each warp's stores are whole 128-byte lines (one lane per line left every 32-byte sector
         // half written: 108 us for the 8192^2 bf16 term, 3.4 TB/s); the padded pitch keeps both
         // passes free of bank conflicts but for the 2-way ones of the reads.
-        __global__ void __launch_bounds__(256) split_transpose(const float *__restrict__ b, unsigned long long ldb, Terms out,
-                                                               int terms, unsigned long long k, unsigned long long n,
-                                                               unsigned long long kp) {
+        __device__ __forceinline__ void split_columns(const SplitJob &job, int terms, unsigned block, float (*tile)[65]) {
+            const unsigned long long across = (job.lines + 63) / 64, tiles = across * (job.kp / 64);
+            const bool vector = job.ld % 4 == 0 && reinterpret_cast<unsigned long long>(job.from) % 16 == 0;
+            for (unsigned long long t = block; t < tiles; t += job.blocks) {
+                const unsigned long long k0 = t / across * 64, n0 = (t - t / across * across) * 64;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const unsigned idx = threadIdx.x + 256u * u, kr = idx / 16, nv = idx % 16;
+                    const unsigned long long kk = k0 + kr, nn = n0 + 4 * nv;
+                    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                    if (kk < job.k) {
+                        const float *src = job.from + kk * job.ld + nn;
+                        if (vector && nn + 4 <= job.lines) {
+                            const float4 q = *reinterpret_cast<const float4 *>(src);
+                            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) v[e] = nn + e < job.lines ? src[e] : 0.0f;
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) tile[kr][4 * nv + e] = v[e];
+                }
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    // eight lanes per output line: a warp writes four lines' 128 contiguous bytes each
+                    const unsigned idx = threadIdx.x + 256u * u, nr = idx / 8, kv = idx % 8;
+                    if (n0 + nr >= job.lines) continue;
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = tile[8 * kv + e][nr];
+                    split_eight(v, terms, job.out, (n0 + nr) * job.kp + k0 + 8 * kv);
+                }
+                __syncthreads();
+            }
+        }
+
+        // Both operands in one launch (a launch of its own for each took 4 to 7 us at orders around 1000, most of it
+        // starting and ending): the first blocks convert A, the others B. It also clears the tickets of
+        // a product whose depth is split.
+        __global__ void __launch_bounds__(256) split_operands(const __grid_constant__ SplitJob a, const __grid_constant__ SplitJob b,
+                                                              int terms, unsigned *tickets, unsigned ticket_count) {
             __shared__ float tile[64][65];
             follow_previous();
-            const unsigned long long k0 = blockIdx.y * 64ull, n0 = blockIdx.x * 64ull;
-            const bool vector = ldb % 4 == 0 && reinterpret_cast<unsigned long long>(b) % 16 == 0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const unsigned idx = threadIdx.x + 256u * u, kr = idx / 16, nv = idx % 16;
-                const unsigned long long kk = k0 + kr, nn = n0 + 4 * nv;
-                float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                if (kk < k) {
-                    const float *src = b + kk * ldb + nn;
-                    if (vector && nn + 4 <= n) {
-                        const float4 q = *reinterpret_cast<const float4 *>(src);
-                        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] = nn + e < n ? src[e] : 0.0f;
-                    }
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) tile[kr][4 * nv + e] = v[e];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                // eight lanes per output row: a warp writes four rows' 128 contiguous bytes each
-                const unsigned idx = threadIdx.x + 256u * u, nr = idx / 8, kv = idx % 8;
-                if (n0 + nr >= n) continue;
-                float v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = tile[8 * kv + e][nr];
-                split_eight(v, terms, out, (n0 + nr) * kp + k0 + 8 * kv);
-            }
+            if (blockIdx.x == 0)
+                for (unsigned i = threadIdx.x; i < ticket_count; i += 256) tickets[i] = 0u;
+            const bool second = blockIdx.x >= a.blocks;
+            const SplitJob &job = second ? b : a;
+            const unsigned block = second ? blockIdx.x - a.blocks : blockIdx.x;
+            if (job.transposed) split_columns(job, terms, block, tile);
+            else split_lines(job, terms, block);
         }
 
         // ---- PTX helpers (tcgen05 / TMA / mbarrier), sm_100a ---------------------------------------
@@ -204,6 +226,10 @@ namespace sci_cuda {
             unsigned long long m, n, kp, ldc;
             int subtract;  // C -= A B instead of C = A B
             int *status;
+            // the pair kernel's split depth: pieces of `span` k-blocks, their sums in `partial`, a ticket per tile and warp
+            unsigned pieces, span;
+            float *partial;
+            unsigned *tickets;
         };
 
         // The bf16 term products a tensor-core tile accumulates: (i, j) multiplies term i of A by term
@@ -391,6 +417,14 @@ namespace sci_cuda {
         // bounded: a role whose wait runs out records the timeout in the status word and stops; the
         // others' waits then run out too, and the pair meets at a cluster barrier before freeing its
         // tensor memory.
+        //
+        // Split depth. A product of few tiles leaves most pairs idle (24 tiles of 74 pairs at 1000 x 700 x 1300), so
+        // its depth is cut into `pieces`, each with every tile: work items are (tile, piece). A piece's
+        // sums go to `partial`; the warp that brings a tile's last piece (a ticket per tile, rank and
+        // warp: a warp only needs its own rows) adds the pieces in their order and writes C, so the
+        // result does not depend on which piece was last. With the operands converted in one launch,
+        // and the product's start beside the conversion's end: split3 1000 x 700 x 1300 42 -> 29 us,
+        // 100 x 3000 x 2000 54 -> 35, bf16 500 x 500 x 4000 41 -> 34, split3 2000^3 97 -> 90.
         constexpr unsigned kGroup = 8;
         constexpr int kSegment = 32;  // k-blocks (64 deep) per segment of the split modes
         template <int TERMS> struct PairShape {
@@ -479,10 +513,16 @@ namespace sci_cuda {
             const unsigned warp = threadIdx.x / 32, lane = threadIdx.x % 32;
             const unsigned rank = pair_rank();
             const unsigned pair = blockIdx.x / 2, pairs = gridDim.x / 2;
-            const unsigned tiles = tiles_m * tiles_n;
-            const int kblocks = static_cast<int>(args.kp / kBK);
-            const int per_segment = Sh::split ? kSegment : kblocks;
-            const int segments = (kblocks + per_segment - 1) / per_segment;
+            const unsigned tiles = tiles_m * tiles_n, items = tiles * args.pieces;
+            const int all_blocks = static_cast<int>(args.kp / kBK);
+            const int per_segment = Sh::split ? kSegment : all_blocks;
+            // item t: tile t % tiles, k-blocks [first, last) of its piece
+            auto item = [&](unsigned t, unsigned &tile, int &first, int &last) {
+                const unsigned piece = t / tiles;
+                tile = t - piece * tiles;
+                first = static_cast<int>(piece * args.span);
+                last = first + static_cast<int>(args.span) < all_blocks ? first + static_cast<int>(args.span) : all_blocks;
+            };
 
             if (threadIdx.x == 0) {
                 for (int s = 0; s < S; ++s) {
@@ -504,6 +544,7 @@ namespace sci_cuda {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             pair_sync();  // both CTAs' barriers exist before either sees a remote arrival or a transfer
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            follow_previous();  // the operands' conversion
             const unsigned tmem = tmem_slot;
 
             if (warp == 4) {
@@ -511,11 +552,13 @@ namespace sci_cuda {
                     // producer: this CTA's 128 rows of A and BN / 2 rows of B^T per term, per stage
                     unsigned s = 0, phase = 0;
                     bool ok = true;
-                    for (unsigned t = pair; t < tiles && ok; t += pairs) {
-                        unsigned tm, tn;
-                        pair_tile(t, tiles_m, tiles_n, tm, tn);
+                    for (unsigned t = pair; t < items && ok; t += pairs) {
+                        unsigned tile, tm, tn;
+                        int first, last;
+                        item(t, tile, first, last);
+                        pair_tile(tile, tiles_m, tiles_n, tm, tn);
                         const int ya = static_cast<int>(tm * 256 + rank * 128), yb = static_cast<int>(tn * BN + rank * (BN / 2));
-                        for (int kb = 0; kb < kblocks && ok; ++kb) {
+                        for (int kb = first; kb < last && ok; ++kb) {
                             if (!mbar_wait(&empty[s], phase ^ 1u)) {
                                 ok = false;
                                 break;
@@ -542,8 +585,11 @@ namespace sci_cuda {
                     // MMA issuer: 256 x BN x 16 steps into the accumulators of buffer b for work item i
                     unsigned s = 0, phase = 0, i = 0;
                     bool ok = true;
-                    for (unsigned t = pair; t < tiles && ok; t += pairs) {
-                        for (int segment = 0; segment < segments && ok; ++segment, ++i) {
+                    for (unsigned t = pair; t < items && ok; t += pairs) {
+                        unsigned tile;
+                        int first_block, last_block;
+                        item(t, tile, first_block, last_block);
+                        for (int k0 = first_block; k0 < last_block && ok; k0 += per_segment, ++i) {
                             const unsigned b = i & 1u;
                             if (!mbar_wait(&acc_empty[b], ((i >> 1) & 1u) ^ 1u)) {
                                 ok = false;
@@ -551,8 +597,7 @@ namespace sci_cuda {
                             }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             const unsigned lead = tmem + b * Sh::buffer, rest = Sh::split ? lead + BN : lead;
-                            const int k0 = segment * per_segment;
-                            const int k1 = k0 + per_segment < kblocks ? k0 + per_segment : kblocks;
+                            const int k1 = k0 + per_segment < last_block ? k0 + per_segment : last_block;
                             for (int kb = k0; kb < k1; ++kb) {
                                 if (!mbar_wait(&full[s], phase)) {
                                     ok = false;
@@ -594,12 +639,16 @@ namespace sci_cuda {
                 const bool vector = (args.ldc % 4) == 0 && (reinterpret_cast<unsigned long long>(args.c) % 16) == 0;
                 unsigned i = 0;
                 bool ok = true;
-                for (unsigned t = pair; t < tiles && ok; t += pairs) {
-                    unsigned tm, tn;
-                    pair_tile(t, tiles_m, tiles_n, tm, tn);
+                for (unsigned t = pair; t < items && ok; t += pairs) {
+                    unsigned tile, tm, tn;
+                    int first, last;
+                    item(t, tile, first, last);
+                    pair_tile(tile, tiles_m, tiles_n, tm, tn);
                     const unsigned long long row = 256ull * tm + 128 * rank + warp * 32 + lane;
                     const unsigned long long n0 = 1ull * tn * BN;
-                    for (int segment = 0; segment < segments; ++segment, ++i) {
+                    // this warp's rows of the piece's sums, BN wide
+                    float *const part = args.partial + ((1ull * t * 2 + rank) * 128 + warp * 32) * BN;
+                    for (int k0 = first; k0 < last; k0 += per_segment, ++i) {
                         const unsigned b = i & 1u;
                         const bool waited = mbar_wait(&acc_full[b], (i >> 1) & 1u);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -610,7 +659,7 @@ namespace sci_cuda {
                         }
                         // the first segment of a product stores; later ones (and every segment of a
                         // subtracting update) combine with what C holds
-                        const int how = args.subtract ? -1 : (segment == 0 ? 0 : 1);
+                        const int how = args.subtract ? -1 : (k0 == first ? 0 : 1);
 #pragma unroll 1
                         for (int chunk = 0; chunk < BN / 32; ++chunk) {
                             unsigned v[32];
@@ -627,7 +676,21 @@ namespace sci_cuda {
                                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                             }
                             const unsigned long long col = n0 + chunk * 32;
-                            if (row < args.m && col < args.n) {
+                            if (args.pieces > 1) {
+                                if (row < args.m && col < args.n) {
+                                    float *dst = part + lane * BN + chunk * 32;
+#pragma unroll
+                                    for (int j = 0; j < 32; j += 4) {
+                                        float4 out = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
+                                                                 __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
+                                        if (k0 != first) {
+                                            const float4 old = *reinterpret_cast<const float4 *>(dst + j);
+                                            out = make_float4(old.x + out.x, old.y + out.y, old.z + out.z, old.w + out.w);
+                                        }
+                                        *reinterpret_cast<float4 *>(dst + j) = out;
+                                    }
+                                }
+                            } else if (row < args.m && col < args.n) {
                                 float *dst = args.c + row * args.ldc + col;
                                 if (col + 32 <= args.n && vector) {
 #pragma unroll
@@ -654,6 +717,49 @@ namespace sci_cuda {
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         __syncwarp();
                         if (lane == 0) pair_arrive(b ? empty1 : empty0);
+                    }
+                    if (args.pieces > 1 && ok) {
+                        unsigned ticket = 0;
+                        __threadfence();
+                        __syncwarp();
+                        if (lane == 0) ticket = atomicAdd(&args.tickets[(tile * 2 + rank) * 4 + warp], 1u);
+                        if (__shfl_sync(0xffffffffu, ticket, 0) == args.pieces - 1) {
+                            __threadfence();
+                            // the lanes along a row, sixteen rows' loads of a piece in flight (row by row the loads'
+                            // latency was longer than the product)
+                            constexpr unsigned R = 16;
+#pragma unroll 1
+                            for (unsigned at = 0; at < 32 / R * (BN / 128); ++at) {
+                                const unsigned r0 = at % (32 / R) * R, c = at / (32 / R) * 128 + 4 * lane;
+                                const unsigned long long line0 = 256ull * tm + 128 * rank + warp * 32 + r0, col = n0 + c;
+                                if (col >= args.n) continue;
+                                float4 sum[R];
+#pragma unroll 1
+                                for (unsigned p = 0; p < args.pieces; ++p) {
+                                    const float *from = args.partial + ((1ull * (p * tiles + tile) * 2 + rank) * 128 + warp * 32 + r0) * BN + c;
+                                    float4 q[R];
+#pragma unroll
+                                    for (unsigned r = 0; r < R; ++r)
+                                        if (line0 + r < args.m) q[r] = __ldcg(reinterpret_cast<const float4 *>(from + r * BN));
+#pragma unroll
+                                    for (unsigned r = 0; r < R; ++r)
+                                        sum[r] = p == 0 ? q[r] : make_float4(sum[r].x + q[r].x, sum[r].y + q[r].y, sum[r].z + q[r].z, sum[r].w + q[r].w);
+                                }
+#pragma unroll
+                                for (unsigned r = 0; r < R; ++r) {
+                                    if (line0 + r >= args.m) break;
+                                    float *dst = args.c + (line0 + r) * args.ldc + col;
+                                    if (vector && col + 4 <= args.n) {
+                                        *reinterpret_cast<float4 *>(dst) = sum[r];
+                                    } else {
+                                        const float out[4] = {sum[r].x, sum[r].y, sum[r].z, sum[r].w};
+#pragma unroll
+                                        for (int e = 0; e < 4; ++e)
+                                            if (col + e < args.n) dst[e] = out[e];
+                                    }
+                                }
+                            }
+                        }
                     }
                 }
             }
@@ -766,7 +872,7 @@ namespace sci_cuda {
             return fn;
         }
 
-        // Whether products of 256 rows or more run on the CTA-pair kernel (the default); the
+        // Whether products that have the GPU to themselves run on the CTA-pair kernel (the default); the
         // environment variable SCI_CUDA_PRODUCT_PAIR=0 keeps them on the one-CTA kernel.
         bool pair_kernel_enabled() {
             static const bool enabled = [] {
@@ -838,7 +944,35 @@ namespace sci_cuda {
         if (kp > (1ull << 31) || m > (1ull << 31) || n > (1ull << 31))
             return ctx.fail(SCI_CUDA_ERROR_UNSUPPORTED, "product dimensions beyond 2^31");
         const unsigned long long a_bytes = (m * kp * 2 + 1023) / 1024 * 1024, b_bytes = (n * kp * 2 + 1023) / 1024 * 1024;
-        const unsigned long long need = terms * (a_bytes + b_bytes) + 1024;
+        // The pair kernel's tiles, and the pieces their depth is cut into: as many as give every pair an item, as long as
+        // that is quicker. A k-block takes about 0.13 us per product of terms and the last warp's pass over
+        // one piece's tile about 0.75 us, so span / pieces x products x 0.13 + pieces x 0.75 is least
+        // where pieces^2 = span x products / 6. (bf16 500 x 500 x 4000, four tiles: 41 us in one piece, 53 in 15.)
+        const bool paired = whole_gpu && pair_kernel_enabled();
+        const unsigned pair_bn = terms == 1 ? PairShape<1>::BN : PairShape<3>::BN;
+        unsigned tiles_m = static_cast<unsigned>((m + 255) / 256), tiles_n = static_cast<unsigned>((n + pair_bn - 1) / pair_bn);
+        const void *pair_kernel = terms == 1 ? reinterpret_cast<const void *>(&tensor_product_pair<1>)
+                                : terms == 2 ? reinterpret_cast<const void *>(&tensor_product_pair<2>)
+                                             : reinterpret_cast<const void *>(&tensor_product_pair<3>);
+        const size_t pair_smem = terms == 1 ? PairShape<1>::stages * PairShape<1>::stage + 1024
+                               : terms == 2 ? PairShape<2>::stages * PairShape<2>::stage + 1024
+                                            : PairShape<3>::stages * PairShape<3>::stage + 1024;
+        const unsigned long long tiles = 1ull * tiles_m * tiles_n;
+        unsigned long long slots = 0, pieces = 1, span = kp / kBK;
+        if (paired) {
+            if (int code = ctx.check(cudaFuncSetAttribute(pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          static_cast<int>(pair_smem)),
+                                     "raising the pair kernel's shared memory"))
+                return code;
+            slots = pair_slots(pair_kernel, pair_smem, ctx.sms);
+            const unsigned long long products = terms == 1 ? 1 : (terms == 2 ? 3 : 6);
+            while (!subtract && (pieces + 1) * tiles <= slots && 6 * (pieces + 1) * (pieces + 1) <= span * products) ++pieces;
+            span = (span + pieces - 1) / pieces;
+            pieces = (kp / kBK + span - 1) / span;
+        }
+        const unsigned long long tile_bytes = 256ull * pair_bn * 4;
+        const unsigned long long partial_bytes = pieces > 1 ? tiles * pieces * tile_bytes + tiles * 8 * 4 : 0;
+        const unsigned long long need = terms * (a_bytes + b_bytes) + partial_bytes + 2048;
         if (int code = ctx.check(ctx.workspace->reserve(need), "reserving the product workspace")) return code;
         auto *base = static_cast<unsigned char *>(ctx.workspace->memory);
         Terms at{}, bt{};
@@ -846,10 +980,13 @@ namespace sci_cuda {
             at.t[q] = reinterpret_cast<__nv_bfloat16 *>(base + q * a_bytes);
             bt.t[q] = reinterpret_cast<__nv_bfloat16 *>(base + terms * a_bytes + q * b_bytes);
         }
-        // chained: launched with programmatic stream serialization (the kernels start with
-        // follow_previous), else the ordinary way
-        auto launch = [&](const void *kernel, dim3 grid, dim3 block, void **params, size_t smem) -> cudaError_t {
-            if (!chained) return cudaLaunchKernel(kernel, grid, block, params, smem, ctx.stream);
+        auto *partial = reinterpret_cast<float *>(base + terms * (a_bytes + b_bytes));
+        unsigned *tickets = reinterpret_cast<unsigned *>(reinterpret_cast<unsigned char *>(partial) + tiles * pieces * tile_bytes);
+        unsigned ticket_count = pieces > 1 ? static_cast<unsigned>(tiles * 8) : 0u;
+        // follows: launched with programmatic stream serialization (the kernels wait for the one before them themselves, and
+        // start beside its end), else the ordinary way
+        auto launch = [&](const void *kernel, dim3 grid, dim3 block, void **params, size_t smem, bool follows) -> cudaError_t {
+            if (!follows) return cudaLaunchKernel(kernel, grid, block, params, smem, ctx.stream);
             cudaLaunchConfig_t config{};
             config.gridDim = grid;
             config.blockDim = block;
@@ -862,51 +999,33 @@ namespace sci_cuda {
             config.numAttrs = 1;
             return cudaLaunchKernelExC(&config, kernel, params);
         };
-        auto rows_of = [&](const float *x, unsigned long long ld, Terms out, unsigned long long rows) {
-            const unsigned grid =
-                    static_cast<unsigned>(std::min<unsigned long long>((rows * (kp / 8) + 255) / 256, ctx.sms * 16ull));
-            int count = terms;
-            unsigned long long kk = k, kpp = kp;
-            void *params[] = {&x, &ld, &out, &count, &rows, &kk, &kpp};
-            return launch(reinterpret_cast<const void *>(&split_rows), dim3(grid), dim3(256), params, 0);
+        auto job = [&](const float *x, unsigned long long ld, Terms out, unsigned long long lines, bool transposed) {
+            const unsigned long long blocks = transposed ? (lines + 63) / 64 * (kp / 64)
+                                                         : std::min<unsigned long long>((lines * (kp / 8) + 255) / 256, ctx.sms * 16ull);
+            return SplitJob{x, ld, lines, k, kp, out, transposed ? 1 : 0,
+                            static_cast<unsigned>(std::min<unsigned long long>(blocks, 1u << 30))};
         };
-        auto columns_of = [&](const float *x, unsigned long long ld, Terms out, unsigned long long columns) {
-            const dim3 tgrid(static_cast<unsigned>((columns + 63) / 64), static_cast<unsigned>(kp / 64));
-            int count = terms;
-            unsigned long long kk = k, kpp = kp;
-            void *params[] = {&x, &ld, &out, &count, &kk, &columns, &kpp};
-            return launch(reinterpret_cast<const void *>(&split_transpose), tgrid, dim3(256), params, 0);
-        };
-        if (int code = ctx.check(a_t ? columns_of(a, lda, at, m) : rows_of(a, lda, at, m), "launching the bf16 conversion"))
-            return code;
-        if (int code = ctx.check(b_t ? rows_of(b, ldb, bt, n) : columns_of(b, ldb, bt, n), "launching the bf16 conversion"))
+        SplitJob job_a = job(a, lda, at, m, a_t), job_b = job(b, ldb, bt, n, !b_t);
+        int term_count = terms;
+        void *split_params[] = {&job_a, &job_b, &term_count, &tickets, &ticket_count};
+        if (int code = ctx.check(launch(reinterpret_cast<const void *>(&split_operands), dim3(job_a.blocks + job_b.blocks), dim3(256),
+                                        split_params, 0, chained),
+                                 "launching the bf16 conversion"))
             return code;
 
-        ProductArgs args{c, m, n, kp, ldc, subtract ? 1 : 0, ctx.status};
-        if (whole_gpu && m >= 256 && pair_kernel_enabled()) {
+        ProductArgs args{c, m, n, kp, ldc, subtract ? 1 : 0, ctx.status, static_cast<unsigned>(pieces), static_cast<unsigned>(span),
+                         partial, tickets};
+        if (paired) {
             // 256 x 256 (one term) or 256 x 128 tiles on CTA pairs, persistent
             Maps maps;
             std::memset(&maps, 0, sizeof(maps));
             for (int q = 0; q < terms; ++q) {
-                const unsigned b_box = terms == 1 ? PairShape<1>::BN / 2 : PairShape<3>::BN / 2;
-                if (!make_map(&maps.a[q], at.t[q], m, kp, 128) || !make_map(&maps.b[q], bt.t[q], n, kp, b_box))
+                if (!make_map(&maps.a[q], at.t[q], m, kp, 128) || !make_map(&maps.b[q], bt.t[q], n, kp, pair_bn / 2))
                     return ctx.fail(SCI_CUDA_ERROR_LAUNCH, "cuTensorMapEncodeTiled failed");
             }
-            const void *kernel = terms == 1 ? reinterpret_cast<const void *>(&tensor_product_pair<1>)
-                               : terms == 2 ? reinterpret_cast<const void *>(&tensor_product_pair<2>)
-                                            : reinterpret_cast<const void *>(&tensor_product_pair<3>);
-            const size_t smem = terms == 1 ? PairShape<1>::stages * PairShape<1>::stage + 1024
-                              : terms == 2 ? PairShape<2>::stages * PairShape<2>::stage + 1024
-                                           : PairShape<3>::stages * PairShape<3>::stage + 1024;
-            if (int code = ctx.check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                                     "raising the pair kernel's shared memory"))
-                return code;
-            const unsigned bn = terms == 1 ? PairShape<1>::BN : PairShape<3>::BN;
-            unsigned tiles_m = static_cast<unsigned>((m + 255) / 256), tiles_n = static_cast<unsigned>((n + bn - 1) / bn);
-            const unsigned long long tiles = 1ull * tiles_m * tiles_n;
-            const unsigned long long pairs = std::min<unsigned long long>(tiles, pair_slots(kernel, smem, ctx.sms));
+            const unsigned long long pairs = std::min<unsigned long long>(tiles * pieces, slots);
             void *params[] = {&maps, &args, &tiles_m, &tiles_n};
-            return ctx.check(cudaLaunchKernel(kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(192), params, smem, ctx.stream),
+            return ctx.check(launch(pair_kernel, dim3(static_cast<unsigned>(2 * pairs)), dim3(192), params, pair_smem, true),
                              "launching the pair tensor product");
         }
 
@@ -928,7 +1047,7 @@ namespace sci_cuda {
             return code;
         void *params[] = {&maps, &args};
         const dim3 pgrid(static_cast<unsigned>((n + bn - 1) / bn), static_cast<unsigned>((m + kBM - 1) / kBM));
-        return ctx.check(launch(kernel, pgrid, dim3(192), params, smem), "launching the tensor product");
+        return ctx.check(launch(kernel, pgrid, dim3(192), params, smem, chained), "launching the tensor product");
     }
 
     // C (pitch ldc) = or -= A (pitch lda) * B (pitch ldb) with the plain SIMT kernel; a_t / b_t as for
