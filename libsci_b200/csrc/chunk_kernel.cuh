@@ -55,6 +55,20 @@ namespace sci_cuda {
         unsigned int ticket;
     };
 
+    // Where the host waits for a reduction: pinned host memory that the last block writes after the
+    // result, the launch's status word and then the word the host polls. A null word: nobody polls.
+    struct Notice {
+        unsigned *word;
+        int *status;
+        unsigned value;
+    };
+    __device__ __forceinline__ void notify(const Notice &notice, const int *status) {
+        if (notice.word == nullptr) return;
+        *notice.status = __ldcg(status);
+        __threadfence_system();  // the result and the status before the word
+        *static_cast<volatile unsigned *>(notice.word) = notice.value;
+    }
+
     // Everything one launch needs, passed by value as a __grid_constant__ parameter (about
     // 1.5 KB), so the launch is self-contained and can be captured into a CUDA graph.
     template <typename T> struct Launch {
@@ -73,8 +87,9 @@ namespace sci_cuda {
         unsigned long long count;
         unsigned long long tail_start;  // elements from here on take the one-lane Scalar forms
         ReduceState *state;
-        double *destination;       // where the folded value is written (device memory)
+        double *destination;       // where the folded value is written (device or pinned host memory)
         int *status;
+        Notice notice;
     };
 
     // ---- the two programs --------------------------------------------------------------------------
@@ -514,13 +529,14 @@ namespace sci_cuda {
     // The grid-wide end of a single-pass fold: each thread's state folds across its warp (shuffle)
     // and block, every block writes one partial, and the last block to take a ticket folds the
     // partials in block order and writes the value to `destination`. Every thread of the block
-    // calls it.
+    // calls it. A block that is alone writes its value at once: the partial, the ticket and the partial's way back
+    // took about half of such a launch.
     template <typename T>
-    // `status`, when given, is the launch's error word: if a block gave up on its copies (its
+    // `status` is the launch's error word: if a block gave up on its copies (its
     // partial then covers only the tiles before it stopped), the result is a quiet NaN instead of a
     // partial fold, so a caller that never reads the word still cannot take the value for a result.
     __device__ __forceinline__ void finish_fold(Fold fold, unsigned op, ReduceState *state, double *destination,
-                                                const int *status = nullptr) {
+                                                const int *status, const Notice &notice) {
         __shared__ double block_total[32];
         __shared__ unsigned block_magnitude[32];
         __shared__ bool last_block;
@@ -545,11 +561,21 @@ namespace sci_cuda {
                 total = combine(op, total, block_total[i]);
                 magnitude = max(magnitude, block_magnitude[i]);
             }
-            state->partial[blockIdx.x] = total;
-            state->poisoned[blockIdx.x] = magnitude > nan_floor<T>() ? 1 : 0;
-            __threadfence();
-            const unsigned ticket = atomicAdd(&state->ticket, 1u);
-            last_block = ticket == gridDim.x - 1;
+            if (gridDim.x == 1) {
+                const double start = op == 0 ? 0.0 : (op == 1 ? __longlong_as_double(0x7ff0000000000000ll)
+                                                              : __longlong_as_double((long long)0xfff0000000000000ull));
+                const bool gave_up = (__ldcg(status) & kStatusTimeout) != 0;
+                *destination = magnitude > nan_floor<T>() || gave_up ? __longlong_as_double(0x7ff8000000000000ll)
+                                                                     : combine(op, start, total);
+                notify(notice, status);
+                last_block = false;
+            } else {
+                state->partial[blockIdx.x] = total;
+                state->poisoned[blockIdx.x] = magnitude > nan_floor<T>() ? 1 : 0;
+                __threadfence();
+                const unsigned ticket = atomicAdd(&state->ticket, 1u);
+                last_block = ticket == gridDim.x - 1;
+            }
         }
         __syncthreads();
         if (last_block && t < 32) {
@@ -570,9 +596,10 @@ namespace sci_cuda {
             }
             if (t == 0) {
                 // every block's atomicOr on the word came before its ticket (fenced), so it is seen here
-                const bool gave_up = status != nullptr && (__ldcg(status) & kStatusTimeout) != 0;
-                *destination = poisoned || gave_up ? __longlong_as_double(0x7ff8000000000000ll) : total;
+                const bool gave_up = (__ldcg(status) & kStatusTimeout) != 0;
                 state->ticket = 0;
+                *destination = poisoned || gave_up ? __longlong_as_double(0x7ff8000000000000ll) : total;
+                notify(notice, status);
             }
         }
     }
@@ -672,7 +699,7 @@ namespace sci_cuda {
             if constexpr (MODE != kEvaluate) fold_tile<T, MODE>(fold, op, value, second, w, false);
         }
 
-        if constexpr (MODE != kEvaluate) finish_fold<T>(fold, op, L.state, L.destination, L.status);
+        if constexpr (MODE != kEvaluate) finish_fold<T>(fold, op, L.state, L.destination, L.status, L.notice);
     }
 
 } // namespace sci_cuda

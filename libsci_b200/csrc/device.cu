@@ -16,6 +16,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <limits>
@@ -31,6 +33,25 @@ namespace sci_cuda {
         if (code) return code;
         code = check(cudaStreamSynchronize(stream), "synchronizing the stream");
         if (code) return code;
+        return settle();
+    }
+
+    int Context::await_notice() {
+        const auto arrived = [&] { return *static_cast<volatile unsigned *>(notice_word) == notice_value; };
+        const auto limit = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+        bool seen = arrived();
+        while (!seen && std::chrono::steady_clock::now() < limit) {
+            for (int spin = 0; spin < 64 && !seen; ++spin) seen = arrived();
+        }
+        if (!seen) {
+            if (int code = check(cudaStreamSynchronize(stream), "synchronizing the stream")) return code;
+            if (!arrived()) return fail(SCI_CUDA_ERROR_LAUNCH, "a reduction ended without its result");
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);  // the result is read after the word
+        return settle();
+    }
+
+    int Context::settle() {
         // Frees whose work is done.
         for (auto it = retired.begin(); it != retired.end();) {
             if (cudaEventQuery(it->done) == cudaSuccess) {
@@ -166,7 +187,8 @@ namespace sci_cuda {
     // Picks the block size, ring depth and grid for a launch, and launches it.
     template <typename T>
     static int launch(Context &ctx, Launch<T> &L, int mode, double *device_result, const sci_chunk &chunk) {
-        L.destination = device_result ? device_result : ctx.result;
+        L.destination = device_result;
+        if (device_result == ctx.host_result) L.notice = ctx.next_notice();  // a blocking reduction
 
         // A specialised kernel when one is ready for this signature (or compiled now in
         // synchronous mode); the generic interpreter otherwise.
@@ -262,14 +284,16 @@ int sci_cuda_open(uint32_t ordinal, sci_cuda_context **context) {
     // the reduction's result with the status word after it (device and pinned host): a blocking
     // reduction reads both with one copy
     if (cudaMalloc(&ctx->state, sizeof(ReduceState)) != cudaSuccess || cudaMalloc(&ctx->result, kResultBytes) != cudaSuccess ||
-        cudaMallocHost(&ctx->host_result, kResultBytes) != cudaSuccess) {
+        cudaMallocHost(&ctx->host_result, kHostResultBytes) != cudaSuccess) {
         return SCI_CUDA_ERROR_MEMORY;
     }
     ctx->status = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(ctx->result) + sizeof(double));
     ctx->host_status = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(ctx->host_result) + sizeof(double));
     cudaMemsetAsync(ctx->state, 0, sizeof(ReduceState), ctx->stream);
     cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream);
+    ctx->notice_word = reinterpret_cast<unsigned *>(reinterpret_cast<unsigned char *>(ctx->host_result) + kResultBytes);
     *ctx->host_status = 0;
+    *ctx->notice_word = 0;
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return SCI_CUDA_ERROR_DEVICE;
     if (const char *setting = std::getenv("SCI_CUDA_JIT")) {
         ctx->jit_mode = std::strcmp(setting, "0") == 0 ? 0 : (std::strcmp(setting, "sync") == 0 ? 2 : 1);
@@ -501,13 +525,9 @@ int sci_cuda_reduce(sci_cuda_context *context, const sci_chunk *chunk, uint32_t 
         return SCI_CUDA_OK;
     }
     cudaSetDevice(context->device);
-    if (int code = dispatch(*context, *chunk, kReduce, fold, count, nullptr, context->result)) return code;
-    // the result and the status word in one copy
-    if (int code = context->check(cudaMemcpyAsync(context->host_result, context->result, kResultBytes,
-                                                  cudaMemcpyDeviceToHost, context->stream),
-                                  "reading the reduction"))
-        return code;
-    if (int code = context->drain(true)) return code;
+    // the kernel writes the result to pinned host memory, and the host waits for its notice
+    if (int code = dispatch(*context, *chunk, kReduce, fold, count, nullptr, context->host_result)) return code;
+    if (int code = context->await_notice()) return code;
     *result = *context->host_result;
     return SCI_CUDA_OK;
 }

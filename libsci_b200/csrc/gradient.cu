@@ -95,7 +95,7 @@ namespace sci_cuda {
             return SCI_CUDA_OK;
         }
 
-        // Queues one gradient form over `count` elements. `value` (device) receives the sum in the
+        // Queues one gradient form over `count` elements. `value` (pinned host memory) receives the sum in the
         // forward forms, or is null.
         template <typename T>
         int launch_gradient(Context &ctx, const sci_chunk &program, int form, uint64_t count, double seed,
@@ -133,6 +133,8 @@ namespace sci_cuda {
             L.tail_start = count - count % (64 / sizeof(T));  // the reference's loop tails (see device.cu)
             L.state = ctx.state;
             L.destination = value;
+            L.status = ctx.status;
+            if (value) L.notice = ctx.next_notice();
 
             const Specialized *special = ctx.specializer ? ctx.specializer->find(ctx, program, form) : nullptr;
             const int per_thread = special && program.length <= 16 ? static_cast<int>(width) : 1;
@@ -196,16 +198,13 @@ extern "C" int sci_cuda_gradient(sci_cuda_context *context, const sci_chunk *chu
     cudaSetDevice(context->device);
     sci_chunk program;
     if (int code = value_form(*context, *chunk, program)) return code;
-    double *device_value = value ? context->result : nullptr;
-    const int code = chunk->precision == SCI_PRECISION_WIDE
-                             ? gradient<double>(*context, program, count, seed, gradients, device_value, form)
-                             : gradient<float>(*context, program, count, seed, gradients, device_value, form);
+    // the kernel writes the sum to pinned host memory and the host waits for its notice
+    double *sum = value ? context->host_result : nullptr;
+    const int code = chunk->precision == SCI_PRECISION_WIDE ? gradient<double>(*context, program, count, seed, gradients, sum, form)
+                                                            : gradient<float>(*context, program, count, seed, gradients, sum, form);
     if (code || !value) return code;  // without a value the call is only queued
-    if (int c = context->check(cudaMemcpyAsync(context->host_result, context->result, sizeof(double),
-                                               cudaMemcpyDeviceToHost, context->stream),
-                               "reading the sum"))
-        return c;
-    if (int c = context->drain()) return c;
+    // the stored form's second pass follows the one that sums
+    if (int c = form == SCI_GRADIENT_STORED ? context->drain() : context->await_notice()) return c;
     *value = *context->host_result;
     return SCI_CUDA_OK;
 }

@@ -44,6 +44,8 @@ namespace sci_cuda {
         unsigned long long tail_start;
         ReduceState *state;
         double *destination;  // the sum, or null
+        int *status;
+        Notice notice;
     };
 
     // A circular code whose derivative holds the other circular function of its operand.
@@ -406,7 +408,7 @@ namespace sci_cuda {
             }
         }
         if constexpr (forward) {
-            if (L.destination != nullptr) finish_fold<T>(fold, 0u, L.state, L.destination);
+            if (L.destination != nullptr) finish_fold<T>(fold, 0u, L.state, L.destination, L.status, L.notice);
         }
     }
 
