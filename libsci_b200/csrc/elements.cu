@@ -21,12 +21,12 @@
 // bit-identical to the host loop's, whatever the launch shape.
 //
 // Kernel: a persistent grid-stride interpreter. A thread owns 16 contiguous bytes of every input
-// per tile (16 int8 ... 2 int64), read and written as one 128-bit access when the arrays are
-// 16-byte aligned; temporaries live in a shared-memory slot file (16 bytes per thread per
-// temporary), the output slot in registers. Each instruction is a warp-uniform switch. Reductions
-// fold lanes in a 64-bit carrier, then the warp (shuffles) and the block, and one atomic per block
-// lands in the context's 8-byte result word. HBM-bound for the arithmetic codes; the real
-// functions are bound by the FP64 pipe.
+// per tile (16 int8 ... 2 int64; 32 bytes in most reductions), read and written in 128-bit accesses
+// when the arrays are 16-byte aligned; temporaries live in a shared-memory slot file (as many bytes
+// per thread per temporary), the output slot in registers. Each instruction is a warp-uniform switch. Reductions
+// fold lanes in a 64-bit carrier, then the warp (shuffles) and the block; the last block to arrive
+// folds the blocks' partials and writes the value to pinned host memory. HBM-bound for the arithmetic
+// codes (division by its own arithmetic too); the real functions are bound by the FP64 pipe.
 #include "context.hpp"
 
 #include <cuda_runtime.h>
@@ -48,14 +48,16 @@ namespace sci_cuda {
             ElementStep steps[kCapacity];
             unsigned length;
             unsigned result;       // value id reduced (reduce launches)
-            unsigned reduce;       // 0 evaluate, 1 reduce
             unsigned fold;         // SCI_FOLD_*
             unsigned vectors;      // inputs and output are 16-byte aligned
             T constants[kCapacity];
             const T *inputs[kCapacity];
             T *output;
             unsigned long long count;
-            unsigned long long *accumulator;
+            ReduceState *state;               // a reduction's partials (64-bit words) and ticket
+            unsigned long long *destination;  // its value: pinned host memory
+            int *status;
+            Notice notice;
         };
 
         // Arithmetic word: the element's width promoted to at least 32 bits, unsigned, so every
@@ -64,12 +66,45 @@ namespace sci_cuda {
         // Fold carrier: the element widened to 64 bits with its signedness, so order is preserved.
         template <typename T> using Carrier = std::conditional_t<std::is_signed<T>::value, long long, unsigned long long>;
 
+        // |a| / |b|, truncated, for b != 0. Up to 32 bits: the integers enter floating point by their bits (2^23 or 2^52
+        // plus the integer, less the power), |a| + 1/2 is multiplied by an approximate 1 / |b|, and the sum with the power
+        // rounded toward zero leaves the integer part in its low bits. (|a| + 1/2) / |b| is at least 1 / (2 |b|) from
+        // every integer, and the product is off by less: |a| / |b| times 2^-21 for 8 and 16 bits in float (|a| < 2^20),
+        // times 2^-39 for 32 bits in double after one Newton step (|a| < 2^38). 64 bits: the correctly rounded
+        // quotient of two integers below 2^52 cannot round up to an integer it does not reach, so its integer part is
+        // exact; larger ones divide as integers. The integer divisions that the compiler expands took 355 us of
+        // max(a, c) / b over 100 million int32 (244 at the memory's rate), 532 over 200 million int8 (122).
+        __device__ __forceinline__ unsigned divide_short(unsigned a, unsigned b) {
+            const float x = __fsub_rn(__uint_as_float(0x4b000000u | a), 8388607.5f), y = __fsub_rn(__uint_as_float(0x4b000000u | b), 8388608.0f);
+            return __float_as_uint(__fadd_rz(__fmul_rn(x, __fdividef(1.0f, y)), 8388608.0f)) & 0x7fffffu;
+        }
+        __device__ __forceinline__ unsigned divide_word(unsigned a, unsigned b) {
+            const double x = __dsub_rn(__hiloint2double(0x43300000, static_cast<int>(a)), 4503599627370495.5);
+            const double y = __dsub_rn(__hiloint2double(0x43300000, static_cast<int>(b)), 4503599627370496.0);
+            double z;
+            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(z) : "d"(y));
+            z = __fma_rn(z, __fma_rn(-y, z, 1.0), z);
+            return static_cast<unsigned>(__double2loint(__dadd_rz(__dmul_rn(x, z), 4503599627370496.0)));
+        }
+        __device__ __forceinline__ unsigned long long divide_long(unsigned long long a, unsigned long long b) {
+            constexpr unsigned long long power = 0x4330000000000000ull, limit = 1ull << 52;
+            if ((a | b) >= limit) return a / b;
+            const double x = __dsub_rn(__longlong_as_double(static_cast<long long>(power | a)), 4503599627370496.0);
+            const double y = __dsub_rn(__longlong_as_double(static_cast<long long>(power | b)), 4503599627370496.0);
+            return static_cast<unsigned long long>(__double_as_longlong(__dadd_rz(__ddiv_rn(x, y), 4503599627370496.0))) & (limit - 1);
+        }
+        // MIN / -1 wraps to MIN: |MIN| is its own bits.
         template <typename T> __device__ __forceinline__ T quotient(T a, T b) {
-            if (b == T(0)) return T(0);
-            if constexpr (std::is_signed<T>::value) {
-                if (b == T(-1)) return T(Word<T>(0) - Word<T>(a));  // MIN / -1 wraps to MIN
-            }
-            return T(a / b);
+            using W = Word<T>;
+            const bool signs = std::is_signed<T>::value && (a < T(0)) != (b < T(0));
+            const W x = std::is_signed<T>::value && a < T(0) ? W(0) - W(a) : W(a);
+            const W y = std::is_signed<T>::value && b < T(0) ? W(0) - W(b) : W(b);
+            W q;
+            if constexpr (sizeof(T) <= 2) q = divide_short(x, y);
+            else if constexpr (sizeof(T) == 4) q = divide_word(x, y);
+            else q = divide_long(x, y == 0 ? W(1) : y);
+            q = signs ? W(0) - q : q;
+            return b == T(0) ? T(0) : T(q);
         }
 
         template <typename T> __device__ __forceinline__ T from_real(double x) {
@@ -113,14 +148,16 @@ namespace sci_cuda {
             }
         }
 
-        template <typename T> struct ElementLanes {
-            static constexpr int count = 16 / sizeof(T);
+        // Bytes of each input that a thread takes per tile: 16, and 32 in reductions (which only read, so more of
+        // it has to be in flight) of elements wider than a byte.
+        template <typename T, bool REDUCE> struct ElementLanes {
+            static constexpr int vectors = REDUCE && sizeof(T) > 1 ? 2 : 1;
+            static constexpr int count = 16 * vectors / sizeof(T);
         };
 
         // One instruction over a thread's lanes; the switch is warp-uniform and sits outside the
         // lane loop.
-        template <typename T> __device__ __forceinline__ void integer_lanes(int code, const T *a, const T *b, const T *c, T *r) {
-            constexpr int K = ElementLanes<T>::count;
+        template <typename T, int K> __device__ __forceinline__ void integer_lanes(int code, const T *a, const T *b, const T *c, T *r) {
             using W = Word<T>;
             switch (code) {
             case SCI_CODE_COPY:
@@ -173,16 +210,19 @@ namespace sci_cuda {
             }
         }
 
-        template <typename T>
+        template <typename T, int K>
         __device__ __forceinline__ void element_fetch(const ElementLaunch<T> &L, unsigned id, unsigned long long first,
                                                       bool full, const T *slots, const T *out, T *v) {
-            constexpr int K = ElementLanes<T>::count;
+            constexpr int N = 16 / sizeof(T);  // lanes of a 16-byte vector
             const unsigned kind = id & kTypes, slot = id & 63;
             if (kind == kInput) {
                 const T *src = L.inputs[slot] + first;
                 if (full && L.vectors) {
-                    const uint4 word = *reinterpret_cast<const uint4 *>(src);
-                    memcpy(v, &word, 16);
+#pragma unroll
+                    for (int e = 0; e < K; e += N) {
+                        const uint4 word = *reinterpret_cast<const uint4 *>(src + e);
+                        memcpy(v + e, &word, 16);
+                    }
                 } else {
 #pragma unroll
                     for (int e = 0; e < K; ++e) v[e] = first + e < L.count ? src[e] : T(0);
@@ -194,8 +234,11 @@ namespace sci_cuda {
 #pragma unroll
                 for (int e = 0; e < K; ++e) v[e] = out[e];
             } else if (id != kNone) {
-                const uint4 word = *reinterpret_cast<const uint4 *>(slots + (slot * blockDim.x + threadIdx.x) * K);
-                memcpy(v, &word, 16);
+#pragma unroll
+                for (int e = 0; e < K; e += N) {
+                    const uint4 word = *reinterpret_cast<const uint4 *>(slots + ((slot * (K / N) + e / N) * blockDim.x + threadIdx.x) * N);
+                    memcpy(v + e, &word, 16);
+                }
             } else {
 #pragma unroll
                 for (int e = 0; e < K; ++e) v[e] = T(0);
@@ -208,22 +251,30 @@ namespace sci_cuda {
             return y > x ? y : x;
         }
 
+        // The same within the element type.
+        template <typename T> __device__ __forceinline__ T fold_identity_of(unsigned fold) {
+            return fold == SCI_FOLD_MINIMUM ? std::numeric_limits<T>::max() : std::numeric_limits<T>::min();
+        }
         template <typename T> __device__ __forceinline__ Carrier<T> fold_identity(unsigned fold) {
             if (fold == SCI_FOLD_SUM) return Carrier<T>(0);
             if (fold == SCI_FOLD_MINIMUM) return std::numeric_limits<Carrier<T>>::max();
             return std::numeric_limits<Carrier<T>>::min();
         }
 
-        template <typename T> __global__ void element_seed(unsigned long long *accumulator, unsigned fold) {
-            *accumulator = static_cast<unsigned long long>(fold_identity<T>(fold));
-        }
+        // Blocks an SM holds: as many as leave the lanes' values in registers.
+        template <typename T, bool REDUCE> struct ElementBlocks {
+            static constexpr int value = sizeof(T) == 1 ? 4 : (REDUCE ? 4 : (sizeof(T) == 2 ? 6 : 5));
+        };
 
-        template <typename T> __global__ void __launch_bounds__(256) element_stream(const __grid_constant__ ElementLaunch<T> L) {
-            constexpr int K = ElementLanes<T>::count;
+        template <typename T, bool REDUCE>
+        __global__ void __launch_bounds__(256, ElementBlocks<T, REDUCE>::value)
+                element_stream(const __grid_constant__ ElementLaunch<T> L) {
+            constexpr int K = ElementLanes<T, REDUCE>::count, N = 16 / sizeof(T);
             extern __shared__ uint4 element_slots[];
             T *slots = reinterpret_cast<T *>(element_slots);
             const unsigned long long tile = 1ull * K * blockDim.x;
             Carrier<T> total = fold_identity<T>(L.fold);
+            Word<T> low = 0;
             for (unsigned long long base = 1ull * blockIdx.x * tile; base < L.count; base += 1ull * gridDim.x * tile) {
                 const unsigned long long first = base + 1ull * threadIdx.x * K;
                 const bool full = first + K <= L.count;
@@ -233,25 +284,40 @@ namespace sci_cuda {
                 for (unsigned i = 0; i < L.length; ++i) {
                     const ElementStep st = L.steps[i];
                     T a[K], b[K], c[K], r[K];
-                    element_fetch(L, st.a, first, full, slots, out, a);
-                    element_fetch(L, st.b, first, full, slots, out, b);
-                    element_fetch(L, st.c, first, full, slots, out, c);
-                    integer_lanes<T>(st.code, a, b, c, r);
+                    element_fetch<T, K>(L, st.a, first, full, slots, out, a);
+                    element_fetch<T, K>(L, st.b, first, full, slots, out, b);
+                    element_fetch<T, K>(L, st.c, first, full, slots, out, c);
+                    integer_lanes<T, K>(st.code, a, b, c, r);
                     if (st.target == kOutput) {
 #pragma unroll
                         for (int e = 0; e < K; ++e) out[e] = r[e];
                     } else {
-                        uint4 word;
-                        memcpy(&word, r, 16);
-                        *reinterpret_cast<uint4 *>(slots + ((st.target & 63) * blockDim.x + threadIdx.x) * K) = word;
+#pragma unroll
+                        for (int e = 0; e < K; e += N) {
+                            uint4 word;
+                            memcpy(&word, r + e, 16);
+                            *reinterpret_cast<uint4 *>(slots + (((st.target & 63) * (K / N) + e / N) * blockDim.x + threadIdx.x) * N) = word;
+                        }
                     }
                 }
-                if (L.reduce) {
+                if constexpr (REDUCE) {
                     T v[K];
-                    element_fetch(L, L.result, first, full, slots, out, v);
+                    element_fetch<T, K>(L, L.result, first, full, slots, out, v);
+                    // A sum keeps its low bits only (it wraps in the element's width), so it runs in the arithmetic word; an
+                    // extreme runs in the element type.
+                    if (L.fold == SCI_FOLD_SUM) {
+                        Word<T> sum = 0;
 #pragma unroll
-                    for (int e = 0; e < K; ++e)
-                        if (first + e < L.count) total = fold_two<T>(L.fold, total, static_cast<Carrier<T>>(v[e]));
+                        for (int e = 0; e < K; ++e)
+                            if (full || first + e < L.count) sum += static_cast<Word<T>>(v[e]);
+                        low += sum;
+                    } else {
+                        T best = static_cast<T>(fold_identity_of<T>(L.fold));
+#pragma unroll
+                        for (int e = 0; e < K; ++e)
+                            if (full || first + e < L.count) best = (L.fold == SCI_FOLD_MINIMUM ? v[e] < best : v[e] > best) ? v[e] : best;
+                        if (first < L.count) total = fold_two<T>(L.fold, total, static_cast<Carrier<T>>(best));
+                    }
                 } else if (first < L.count) {
                     T *dst = L.output + first;
                     if (full && L.vectors) {
@@ -265,8 +331,9 @@ namespace sci_cuda {
                     }
                 }
             }
-            if (!L.reduce) return;
-            // warp, then block, then one atomic per block
+            if constexpr (!REDUCE) return;
+            if (L.fold == SCI_FOLD_SUM) total = static_cast<Carrier<T>>(low);
+            // warp, then block; each block leaves a partial and the last one to arrive folds them all
 #pragma unroll
             for (int offset = 16; offset > 0; offset >>= 1)
                 total = fold_two<T>(L.fold, total, __shfl_xor_sync(0xffffffffu, total, offset));
@@ -279,16 +346,25 @@ namespace sci_cuda {
 #pragma unroll
                 for (int offset = 16; offset > 0; offset >>= 1)
                     total = fold_two<T>(L.fold, total, __shfl_xor_sync(0xffffffffu, total, offset));
+                bool last = false;
                 if (lane == 0) {
-                    if (L.fold == SCI_FOLD_SUM) {
-                        atomicAdd(L.accumulator, static_cast<unsigned long long>(total));
-                    } else if constexpr (std::is_signed<T>::value) {
-                        long long *word = reinterpret_cast<long long *>(L.accumulator);
-                        if (L.fold == SCI_FOLD_MINIMUM) atomicMin(word, static_cast<long long>(total));
-                        else atomicMax(word, static_cast<long long>(total));
-                    } else {
-                        if (L.fold == SCI_FOLD_MINIMUM) atomicMin(L.accumulator, static_cast<unsigned long long>(total));
-                        else atomicMax(L.accumulator, static_cast<unsigned long long>(total));
+                    auto *partials = reinterpret_cast<unsigned long long *>(L.state->partial);
+                    partials[blockIdx.x] = static_cast<unsigned long long>(total);
+                    __threadfence();
+                    last = atomicAdd(&L.state->ticket, 1u) == gridDim.x - 1;
+                }
+                if (__shfl_sync(0xffffffffu, last ? 1 : 0, 0)) {
+                    __threadfence();
+                    const auto *partials = reinterpret_cast<const unsigned long long *>(L.state->partial);
+                    total = fold_identity<T>(L.fold);
+                    for (unsigned b = lane; b < gridDim.x; b += 32) total = fold_two<T>(L.fold, total, static_cast<Carrier<T>>(__ldcg(partials + b)));
+#pragma unroll
+                    for (int offset = 16; offset > 0; offset >>= 1)
+                        total = fold_two<T>(L.fold, total, __shfl_xor_sync(0xffffffffu, total, offset));
+                    if (lane == 0) {
+                        L.state->ticket = 0;
+                        *L.destination = static_cast<unsigned long long>(total);
+                        notify(L.notice, L.status);
                     }
                 }
             }
@@ -303,7 +379,6 @@ namespace sci_cuda {
             ElementLaunch<T> L{};
             L.length = chunk.length;
             L.result = chunk.result;
-            L.reduce = reducing ? 1 : 0;
             L.fold = fold;
             bool vectors = reducing || aligned16(output);
             for (int i = 0; i < chunk.length; ++i) {
@@ -318,15 +393,18 @@ namespace sci_cuda {
             L.vectors = vectors ? 1 : 0;
             L.output = static_cast<T *>(output);
             L.count = count;
-            L.accumulator = reinterpret_cast<unsigned long long *>(ctx.result);
+            L.state = ctx.state;
+            L.destination = reinterpret_cast<unsigned long long *>(ctx.host_result);
+            L.status = ctx.status;
 
-            const void *kernel = reinterpret_cast<const void *>(&element_stream<T>);
+            const void *kernel = reducing ? reinterpret_cast<const void *>(&element_stream<T, true>)
+                                          : reinterpret_cast<const void *>(&element_stream<T, false>);
+            const int lanes = reducing ? ElementLanes<T, true>::count : ElementLanes<T, false>::count;
             int threads = 256;
-            size_t smem = static_cast<size_t>(chunk.temporaries) * 16 * threads;
-            if (smem > 48 * 1024) {
-                threads = 128;
-                smem = static_cast<size_t>(chunk.temporaries) * 16 * threads;
-            }
+            auto slot_file = [&] { return static_cast<size_t>(chunk.temporaries) * lanes * sizeof(T) * threads; };
+            if (slot_file() > 48 * 1024) threads = 128;
+            while (threads > 64 && slot_file() > ctx.shared_limit) threads /= 2;
+            const size_t smem = slot_file();
             if (smem > 48 * 1024) {
                 if (smem > ctx.shared_limit) return ctx.fail(SCI_CUDA_ERROR_INVALID, "%u temporaries exceed shared memory", chunk.temporaries);
                 if (int code = ctx.check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -334,19 +412,17 @@ namespace sci_cuda {
                                          "element slot file"))
                     return code;
             }
-            const unsigned long long tile = 1ull * ElementLanes<T>::count * threads;
+            const unsigned long long tile = 1ull * lanes * threads;
             const unsigned long long tiles = (count + tile - 1) / tile;
             const unsigned long long most = 1ull * ctx.sms * ctx.blocks_per_sm(kernel, threads, smem);
             const unsigned grid = static_cast<unsigned>(tiles < most ? tiles : most);
-            if (reducing) element_seed<T><<<1, 1, 0, ctx.stream>>>(L.accumulator, fold);
-            element_stream<T><<<grid, threads, smem, ctx.stream>>>(L);
-            if (int code = ctx.check(cudaGetLastError(), "launching an element chunk")) return code;
-            if (!reducing) return SCI_CUDA_OK;
-            if (int code = ctx.check(cudaMemcpyAsync(ctx.host_result, ctx.result, sizeof(double), cudaMemcpyDeviceToHost,
-                                                     ctx.stream),
-                                     "reading the element reduction"))
+            if (reducing) L.notice = ctx.next_notice();
+            void *args[] = {&L};
+            if (int code = ctx.check(cudaLaunchKernel(kernel, dim3(grid), dim3(threads), args, smem, ctx.stream),
+                                     "launching an element chunk"))
                 return code;
-            if (int code = ctx.drain()) return code;
+            if (!reducing) return SCI_CUDA_OK;
+            if (int code = ctx.await_notice()) return code;
             unsigned long long word;
             std::memcpy(&word, ctx.host_result, sizeof(word));
             const T value = static_cast<T>(word);  // low bits: the sum wraps in the element's width
