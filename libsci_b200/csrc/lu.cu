@@ -33,6 +33,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <cstdint>
@@ -2661,28 +2663,39 @@ namespace {
                small_solve_blocks(width, transposed) <= 2u * static_cast<unsigned>(ctx.sms);
     }
 
-    // Waits for a small solve and takes the largest backward error and iteration count of CTAs [first, last).
+    // What a small solve's CTAs report, in pinned memory that they write themselves.
     struct SmallReports {
-        double *errors;
-        int *iterations;
-        unsigned blocks;
-        static unsigned long long bytes(unsigned blocks) { return 12ull * blocks + 16; }
-        int read(Context &ctx) {
-            host = pinned_doubles(ctx, (bytes(blocks) + 7) / 8);
-            if (host == nullptr) return ctx.fail(SCI_CUDA_ERROR_MEMORY, "pinned host memory for the report");
-            if (int code = ctx.check(cudaMemcpyAsync(host, errors, 12ull * blocks, cudaMemcpyDeviceToHost, ctx.stream),
-                                     "reading the small solve's report"))
-                return code;
-            return ctx.drain();
+        double *errors{nullptr};
+        volatile int *iterations{nullptr};
+        unsigned blocks{0};
+        int prepare(Context &ctx, unsigned count) {
+            blocks = count;
+            errors = pinned_doubles(ctx, count + (count + 1) / 2);
+            if (errors == nullptr) return ctx.fail(SCI_CUDA_ERROR_MEMORY, "pinned host memory for the report");
+            iterations = reinterpret_cast<int *>(errors + count);
+            for (unsigned b = 0; b < count; ++b) iterations[b] = 0;  // a CTA takes at least one correction
+            return SCI_CUDA_OK;
+        }
+        // Polls for every CTA's count for a while, then waits for the stream.
+        int wait(Context &ctx) {
+            const auto limit = std::chrono::steady_clock::now() + std::chrono::milliseconds(2);
+            for (unsigned b = 0; b < blocks; ++b) {
+                for (unsigned spin = 1; iterations[b] == 0; ++spin) {
+                    if (spin % 64 != 0 || std::chrono::steady_clock::now() < limit) continue;
+                    if (int code = ctx.check(cudaStreamSynchronize(ctx.stream), "synchronizing the stream")) return code;
+                    if (iterations[b] == 0) return ctx.fail(SCI_CUDA_ERROR_LAUNCH, "a small solve ended without its result");
+                }
+            }
+            std::atomic_thread_fence(std::memory_order_acquire);  // the errors are read after the counts
+            return ctx.settle();
         }
         void largest(unsigned first, unsigned last, double &error, int &count) const {
-            const int *counts = reinterpret_cast<const int *>(host + blocks);
             for (unsigned b = first; b < last; ++b) {
-                error = (host[b] > error || host[b] != host[b]) ? host[b] : error;
-                count = std::max(count, counts[b]);
+                error = (errors[b] > error || errors[b] != errors[b]) ? errors[b] : error;
+                const int own = iterations[b];
+                count = std::max(count, own);
             }
         }
-        double *host{nullptr};
     };
 
     bool overlap(const void *p, unsigned long long p_bytes, const void *q, unsigned long long q_bytes) {
@@ -2709,15 +2722,13 @@ extern "C" int sci_cuda_solve(sci_cuda_context *context, uint32_t precision, uin
     const unsigned long long n = order, nw = order * width;
     if (refine == SCI_REFINE_FP64 && small_solve_fits(*context, n, width, false)) {
         const unsigned blocks = small_solve_blocks(width, false);
-        if (int code = context->check(context->solver->reserve(SmallReports::bytes(blocks)), "reserving the solver workspace"))
-            return code;
-        auto *errors = static_cast<double *>(context->solver->memory);
-        SmallReports reports{errors, reinterpret_cast<int *>(errors + blocks), blocks};
+        SmallReports reports;
+        if (int code = reports.prepare(*context, blocks)) return code;
         if (int code = small_solve_call(*context, static_cast<const double *>(matrix), static_cast<const double *>(right),
                                         static_cast<double *>(solution), nullptr, nullptr, n, width, refinement_target(n),
-                                        reports.errors, reports.iterations))
+                                        reports.errors, const_cast<int *>(reports.iterations)))
             return code;
-        if (int code = reports.read(*context)) return code;
+        if (int code = reports.wait(*context)) return code;
         if (report) reports.largest(0, blocks, report->backward_error, report->iterations);
         return SCI_CUDA_OK;
     }
@@ -2897,17 +2908,15 @@ extern "C" int sci_cuda_solve_gradient(sci_cuda_context *context, uint32_t preci
         !overlap(right_gradient, nw * 8, right, nw * 8) && !overlap(right_gradient, nw * 8, matrix, n * n * 8) &&
         !overlap(right_gradient, nw * 8, solution, nw * 8)) {
         const unsigned blocks = small_solve_blocks(width, true);
-        const unsigned long long space = (SmallReports::bytes(blocks) + 255) / 256 * 256;
-        if (int code = context->check(context->solver->reserve(space + 2 * (nw * 8 + 256)), "reserving the solver workspace"))
-            return code;
-        auto *errors = static_cast<double *>(context->solver->memory);
-        SmallReports reports{errors, reinterpret_cast<int *>(errors + blocks), blocks};
-        auto *spare = reinterpret_cast<double *>(static_cast<unsigned char *>(context->solver->memory) + space);
+        if (int code = context->check(context->solver->reserve(2 * (nw * 8 + 256)), "reserving the solver workspace")) return code;
+        SmallReports reports;
+        if (int code = reports.prepare(*context, blocks)) return code;
+        auto *spare = static_cast<double *>(context->solver->memory);
         double *x = solution ? static_cast<double *>(solution) : spare;
         double *lambda = right_gradient ? static_cast<double *>(right_gradient) : spare + nw;
         if (int code = small_solve_call(*context, static_cast<const double *>(matrix), static_cast<const double *>(right), x,
                                         static_cast<const double *>(upstream), lambda, n, width, refinement_target(n),
-                                        reports.errors, reports.iterations))
+                                        reports.errors, const_cast<int *>(reports.iterations)))
             return code;
         if (matrix_gradient) {
             const unsigned tiles = static_cast<unsigned>((n + 31) / 32);
@@ -2915,7 +2924,7 @@ extern "C" int sci_cuda_solve_gradient(sci_cuda_context *context, uint32_t preci
                                                                             static_cast<unsigned>(n), static_cast<unsigned>(width));
             if (int code = context->check(cudaGetLastError(), "launching the matrix gradient")) return code;
         }
-        if (int code = reports.read(*context)) return code;
+        if (int code = matrix_gradient ? context->drain() : reports.wait(*context)) return code;
         if (report) {
             int forward = 0, transposed = 0;
             reports.largest(0, blocks / 2, report->backward_error, forward);

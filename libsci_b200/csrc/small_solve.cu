@@ -50,7 +50,7 @@ namespace sci_cuda {
                          double *errors, int *iterations) {
         const unsigned blocks = small_solve_blocks(width, b_transposed != nullptr);
         SmallCall call{a, b, b_transposed, x, x_transposed, static_cast<unsigned>(n), static_cast<unsigned>(width),
-                       width == 1 ? 1u : kSmallGroup, small_solve_blocks(width, false)};
+                       width == 1 ? 1u : kSmallGroup, small_solve_blocks(width, false), ctx.status, ctx.host_status};
         const SmallSystem *systems = nullptr;
         const unsigned *order = nullptr;
         void *args[] = {&systems, &order, &call, &target, &errors, &iterations};

@@ -126,6 +126,8 @@ namespace sci_cuda {
         const double *a, *b, *b_transposed;
         double *x, *x_transposed;
         unsigned n, width, group, groups;
+        const int *status;  // the context's error word, and where the first CTA copies it for the host (or null)
+        int *host_status;
         __device__ __forceinline__ SmallSystem system(unsigned block) const {
             const bool flip = block >= groups;
             const unsigned first = (flip ? block - groups : block) * group;
@@ -318,9 +320,13 @@ namespace sci_cuda {
         //  - nothing but the loop branches (10 to 20 cycles each): selects and predicated stores, and the number
         //    of 16-byte pieces a row still has is a constant for eight columns at a time. With branches a column
         //    took 1030 cycles at order 128; all 32 columns unrolled took 840, waiting for instructions.
-        auto columns_of = [&](auto rows_c, auto &w, auto &line, auto &spot, int crew, int j0, int bw, auto home) {
+        auto columns_of = [&](auto rows_c, auto alone_c, auto &w, auto &line, auto &spot, int crew, int j0, int bw, auto home) {
             constexpr int R = decltype(rows_c)::value, kCrew = kWarps / R;
-            auto meet = [&] { asm volatile("bar.sync 1, %0;" ::"r"(32 * crew) : "memory"); };
+            constexpr bool alone = decltype(alone_c)::value != 0;  // a crew of one warp: its maximum is the pivot
+            auto meet = [&] {
+                if constexpr (alone) __syncwarp();
+                else asm volatile("bar.sync 1, %0;" ::"r"(32 * crew) : "memory");
+            };
             static_for<4>([&](auto segment_c) {
                 constexpr int segment = decltype(segment_c)::value, V = 8 - 2 * segment;
 #pragma unroll 1
@@ -353,17 +359,22 @@ namespace sci_cuda {
                         mine = __ballot_sync(kAll, own_key == most && own_place == lowest);
                     }
                     const bool leads = lane == __ffs(mine) - 1;
-                    small_store_if(leads, &best[warp], most, own_place);
-                    meet();
-                    uint2 top = best[0];
+                    uint2 top;
                     int from = 0;
+                    if constexpr (alone) {
+                        top = make_uint2(most, __shfl_sync(kAll, own_place, __ffs(mine) - 1));
+                    } else {
+                        small_store_if(leads, &best[warp], most, own_place);
+                        meet();
+                        top = best[0];
 #pragma unroll
-                    for (int v = 1; v < kCrew; ++v) {
-                        const uint2 other = best[v];
-                        const bool better = other.x > top.x || (other.x == top.x && other.y < top.y);
-                        top.x = better ? other.x : top.x, top.y = better ? other.y : top.y, from = better ? v : from;
+                        for (int v = 1; v < kCrew; ++v) {
+                            const uint2 other = best[v];
+                            const bool better = other.x > top.x || (other.x == top.x && other.y < top.y);
+                            top.x = better ? other.x : top.x, top.y = better ? other.y : top.y, from = better ? v : from;
+                        }
                     }
-                    const bool winner = leads && warp == from;
+                    const bool winner = leads && (alone || warp == from);
                     float *pivot = pivot_rows[j & 1];
 #pragma unroll
                     for (int h = 0; h < R; ++h) {
@@ -444,7 +455,7 @@ namespace sci_cuda {
                 float kept[32];
                 const int line[1] = {tid};
                 int spot[1] = {place};
-                columns_of(Int<1>{}, held_rows, line, spot, warps, j0, bw, [&](int, int, float entry) {
+                columns_of(Int<1>{}, Int<0>{}, held_rows, line, spot, warps, j0, bw, [&](int, int, float entry) {
 #pragma unroll
                     for (int c = 0; c < 31; ++c) kept[c] = kept[c + 1];
                     kept[31] = entry;
@@ -560,9 +571,11 @@ namespace sci_cuda {
                             w[h][c] = v.x, w[h][c + 1] = v.y, w[h][c + 2] = v.z, w[h][c + 3] = v.w;
                         }
                     }
-                    columns_of(Int<2>{}, w, line, spot, crew, j0, bw, [&](int h, int column, float entry) {
+                    auto home = [&](int h, int column, float entry) {
                         if (line[h] < n) A[line[h] * P + column] = entry;
-                    });
+                    };
+                    if (crew == 1) columns_of(Int<2>{}, Int<1>{}, w, line, spot, crew, j0, bw, home);
+                    else columns_of(Int<2>{}, Int<0>{}, w, line, spot, crew, j0, bw, home);
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
                         if (line[h] < n) {
@@ -911,9 +924,16 @@ namespace sci_cuda {
             for (int q = 0; q < NR; ++q)
                 if (q < static_cast<int>(sys.columns)) sys.x[1ull * tid * sys.pitch + q] = x[tid * NR + q];
         }
+        if (call.host_status != nullptr) {
+            // the host polls `iterations`: the solution, the error and the status come before it
+            __threadfence();
+            __syncthreads();
+            if (tid == 0 && blockIdx.x == 0) *call.host_status = __ldcg(call.status);
+        }
         if (tid == 0) {
             if (errors) errors[id] = berr;
-            if (iterations) iterations[id] = count;
+            if (call.host_status != nullptr) __threadfence_system();
+            if (iterations) *static_cast<volatile int *>(iterations + id) = count;
         }
     }
 

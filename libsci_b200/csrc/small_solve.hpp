@@ -16,7 +16,8 @@ namespace sci_cuda {
     int small_solve_table(Context &ctx, cudaStream_t stream, const SmallSystem *systems, const unsigned *order,
                           unsigned count, unsigned most, double target, double *errors, int *iterations);
     // One call's right-hand sides: X of A X = B (n x width) and, with `b_transposed`, of A^T X = B. Queued on the
-    // context's stream; errors / iterations: an entry per CTA (small_solve_blocks).
+    // context's stream; errors / iterations: an entry per CTA (small_solve_blocks), pinned host memory. A CTA's iteration
+    // count is written last, after its part of X and, by the first, the status word in host_status.
     unsigned small_solve_blocks(unsigned long long width, bool transposed);
     int small_solve_call(Context &ctx, const double *a, const double *b, double *x, const double *b_transposed,
                          double *x_transposed, unsigned long long n, unsigned long long width, double target,
