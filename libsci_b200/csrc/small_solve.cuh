@@ -61,7 +61,7 @@ namespace sci_cuda {
     // Dynamic shared memory of one launch for systems up to order `most`.
     inline unsigned long long small_shared_bytes(int most, int right_sides, int register_blocks) {
         unsigned long long bytes = 4ull * most * small_pitch(most, register_blocks);  // factors
-        bytes += 2ull * 32 * kSmallPitch * 4;                    // published blocks (later: residuals)
+        bytes += 2ull * 32 * kSmallPitch * 4;                    // published blocks (later: products with x)
         bytes += 4ull * register_blocks * 32 * kSmallPitch;      // inverses of register blocks
         bytes += 8ull * most * right_sides;                      // x
         bytes += 2ull * 2 * most;                                // rows by position, positions by row
@@ -164,7 +164,7 @@ namespace sci_cuda {
         unsigned char *cursor = small_shared + 4ull * n * P;
         float *published = reinterpret_cast<float *>(cursor);  // the block's rows as they were
         float *u_block = published + 32 * kSmallPitch;         // and as rows of U (or a block's L and U to invert)
-        double *r = reinterpret_cast<double *>(cursor);        // residuals, once the factors are done
+        double *sums = reinterpret_cast<double *>(cursor);     // the rows' products with x, once the factors are done
         cursor += 2ull * 32 * kSmallPitch * 4;
         float *inverses = reinterpret_cast<float *>(cursor);
         cursor += 4ull * RB * 32 * kSmallPitch;
@@ -813,9 +813,9 @@ namespace sci_cuda {
                 if (at < 0) subtract(l);
             }
             // r = b - A x in FP64, with |r_q|_inf and |x_q|_inf
-            double r_max[NR], x_max[NR];
+            double left[NR], r_max[NR], x_max[NR];  // this row's residuals
 #pragma unroll
-            for (int q = 0; q < NR; ++q) r_max[q] = 0.0;
+            for (int q = 0; q < NR; ++q) left[q] = 0.0;
             if (sys.transposed) {
                 if (row) {
                     double s[NR][2];
@@ -837,9 +837,7 @@ namespace sci_cuda {
                     }
 #pragma unroll
                     for (int q = 0; q < NR; ++q) {
-                        const double residual = rhs[q] - (s[q][0] + s[q][1]);
-                        r[tid * NR + q] = residual;
-                        r_max[q] = fabs(residual);
+                        left[q] = rhs[q] - (s[q][0] + s[q][1]);
                     }
                 }
             } else {
@@ -875,23 +873,22 @@ namespace sci_cuda {
                         int which;
                         const double total = small_warp_sums<M>(s, lane, which);
                         const int at = row0 + which / NR * warps, q = which % NR;
-                        if (at < n && lane % (32 / M) == 0) {
-                            const double value = q < static_cast<int>(sys.columns) ? sys.b[1ull * at * sys.pitch + q] : 0.0;
-                            const double left = value - total;
-                            r[at * NR + q] = left;
-#pragma unroll
-                            for (int p = 0; p < NR; ++p)
-                                if (p == q) r_max[p] = small_larger(fabs(left), r_max[p]);
-                        }
+                        if (at < n && lane % (32 / M) == 0) sums[at * NR + q] = total;
                     }
                 };
                 if (nb == 1) residual(Int<1>{});
                 else if (nb == 2) residual(Int<2>{});
                 else if (nb <= 4) residual(Int<4>{});
                 else residual(Int<8>{});
+                __syncthreads();
+                if (row) {
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) left[q] = rhs[q] - sums[tid * NR + q];
+                }
             }
 #pragma unroll
             for (int q = 0; q < NR; ++q) {
+                r_max[q] = fabs(left[q]);
                 x_max[q] = row ? fabs(x[tid * NR + q]) : 0.0;
 #pragma unroll
                 for (int offset = 16; offset > 0; offset >>= 1) {
@@ -914,10 +911,8 @@ namespace sci_cuda {
             ++count;
             if (count >= 30 || !(berr > target) || !(berr < 0.5 * previous)) break;
             previous = berr;
-            if (row) {
 #pragma unroll
-                for (int q = 0; q < NR; ++q) c[q] = static_cast<float>(r[tid * NR + q]);
-            }
+            for (int q = 0; q < NR; ++q) c[q] = static_cast<float>(left[q]);
         }
         if (row) {
 #pragma unroll
