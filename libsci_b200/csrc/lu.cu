@@ -106,21 +106,39 @@ namespace sci_cuda {
         __device__ __forceinline__ unsigned long long magnitude_key(double m) {
             return static_cast<unsigned long long>(__double_as_longlong(m)) + 1ull;
         }
-        // Every lane of the warp ends with the warp's best (key, row): warp reductions of the key,
-        // then of the row among the lanes that hold the best key.
-        __device__ __forceinline__ void best_of_warp(unsigned &key, unsigned &rel) {
+        // The lane that holds the best (key, row) of the warp: a warp maximum of the key and a vote
+        // for its lane; only equal keys take a minimum of their rows. `key` becomes the best key.
+        __device__ __forceinline__ unsigned key_holders(unsigned &key) {
             const unsigned top = __reduce_max_sync(0xffffffffu, key);
-            rel = __reduce_min_sync(0xffffffffu, key == top ? rel : kNoRow);
+            const unsigned holders = __ballot_sync(0xffffffffu, key == top);
             key = top;
+            return holders;
         }
-        __device__ __forceinline__ void best_of_warp(unsigned long long &key, unsigned &rel) {
+        __device__ __forceinline__ unsigned key_holders(unsigned long long &key) {
             const unsigned hi = static_cast<unsigned>(key >> 32), lo = static_cast<unsigned>(key);
             const unsigned top_hi = __reduce_max_sync(0xffffffffu, hi);
             const unsigned top_lo = __reduce_max_sync(0xffffffffu, hi == top_hi ? lo : 0u);
-            const bool tie = hi == top_hi && lo == top_lo;
-            rel = __reduce_min_sync(0xffffffffu, tie ? rel : kNoRow);
+            const unsigned holders = __ballot_sync(0xffffffffu, hi == top_hi && lo == top_lo);
             key = (static_cast<unsigned long long>(top_hi) << 32) | top_lo;
+            return holders;
         }
+        template <typename K> __device__ __forceinline__ unsigned best_of_warp(K &key, unsigned rel) {
+            const K own = key;
+            unsigned holders = key_holders(key);
+            if (holders & (holders - 1u)) {  // the same for the whole warp
+                const unsigned least = __reduce_min_sync(0xffffffffu, own == key ? rel : kNoRow);
+                holders = __ballot_sync(0xffffffffu, own == key && rel == least);
+            }
+            return static_cast<unsigned>(__ffs(holders)) - 1u;
+        }
+        // A candidate for the pivot: its row's values from the current column on, and the head that the
+        // choice is made by. Rows are below 2^32 (n <= kPanelRows), so origin and position take 32
+        // bits each. The values of one row and the head are 9 16-byte words.
+        template <typename T> struct alignas(16) Candidate {
+            T values[PanelWidth<T>::value];
+            unsigned long long key;
+            unsigned origin, at;  // from the panel's first row: where the row started, where it is now
+        };
         template <int N> struct Span {
             static constexpr int value = N;
         };
@@ -217,47 +235,47 @@ namespace sci_cuda {
         // the current column is always v[i][0] (the column loop stays rolled: unrolled, every column
         // ran cold out of the instruction cache).
         //
-        // Each finished value belongs to the row's original position (`origin`). A multiplier of L
-        // whose row is still at its origin is staged in shared memory and written out coalesced at
-        // the end; one of a row the exchanges moved, and each pivot row of U, goes to global memory
-        // at once. A final permutation moves the at most 2 W displaced rows to their positions.
+        // An exchange moves no values: a row stays in its thread (its origin) and only its position
+        // changes, in the two threads concerned. A row's multipliers of L are staged in shared memory
+        // and written out coalesced at the end, as are the pivot rows of U, at the rows' origins; a
+        // final permutation moves the at most 2 W displaced rows to their positions.
         //
-        // Per column: each warp's best row is published in shared memory; after one CTA barrier,
-        // warp 0 pushes the CTA's candidate with its values into every CTA's inbox (st.async,
-        // counted on the receiver's mbarrier; CTA 0 also pushes the row at the pivot position);
-        // then every warp of every CTA waits for its own inbox to fill (a bounded wait), picks the
-        // pivot from it and eliminates, so the column takes one CTA barrier. A row's next column is
-        // eliminated first and the warp's search for the next pivot issued at once, so the search's
-        // latency overlaps the rest of the elimination. Inboxes and the published candidates
-        // alternate by column parity; a CTA sends into an inbox again only after the barrier of the
-        // column in between, which its warps reach only after reading every message of the earlier
-        // column, and warp 0 reads a parity's candidates before the barrier after which the warps
-        // publish into it again.
+        // Per column: each warp's best row is published in shared memory; after one CTA barrier, up to
+        // four warps (one per scheduler) each reduce the warps' candidates and send the winner to
+        // their share of the CTAs' inboxes (st.async, counted on the receiver's mbarrier); then every
+        // warp of every CTA waits for its own inbox to fill (a bounded wait), picks the pivot from it
+        // and eliminates, so the column takes one CTA barrier. A row's next column is eliminated first
+        // and the warp's search for the next pivot issued at once, so the search's latency overlaps
+        // the rest of the elimination. Inboxes and the published candidates alternate by column
+        // parity; a CTA sends into an inbox again only after the barrier of the column in between,
+        // which its warps reach only after reading every message of the earlier column, and the
+        // senders read a parity's candidates before the barrier after which the warps publish into it
+        // again.
+        //
+        // What bounds it is that chain of latencies, one per column. Measured on the refined solve of
+        // order 8192 (8192 columns in 256 panels): 20.0 ms when an exchange moved the rows' values (a
+        // second message from CTA 0 and scattered stores of the moved rows' multipliers), 19.2 ms with
+        // rows kept in place, 18.8 ms with a message sent by one store whose lanes hold its 16-byte
+        // words (one lane sent all of a CTA's words before). 8 and 16 sending warps: 18.8 ms each;
+        // CTAs of 256 threads with two rows a thread: 7% slower.
         template <typename T, int CL, int ROWS>
         __global__ void __launch_bounds__(kPanelBlock, 1)
                 panel_factor(T *a, unsigned long long n, unsigned long long j0, int width, long long *piv, Movement *moved,
                              int *status) {
             constexpr int kClusterCtas = CL, kCtaRows = PanelShape<CL, ROWS>::rows;
             constexpr int W = PanelWidth<T>::value, R = PanelShape<CL, ROWS>::per_thread, TH = kPanelBlock, WARPS = TH / 32;
+            constexpr unsigned SENDERS = CL < 4 ? CL : 4;
             constexpr int P = kCtaRows + 1;  // pitch of the staged multipliers
             extern __shared__ __align__(16) unsigned char panel_shared[];
             T *stage = reinterpret_cast<T *>(panel_shared);  // stage[k * P + local row]
             __shared__ unsigned home[kCtaRows];          // bit k: stage holds column k of the row
             using Key = typename MagnitudeKey<T>::type;
-            __shared__ Key warp_key[2][WARPS];
-            __shared__ unsigned warp_rel[2][WARPS];
-            __shared__ unsigned long long warp_origin[2][WARPS];
-            __shared__ __align__(16) T warp_values[2][WARPS][W];
-            // The inbox, by column parity: slot q < CL holds CTA q's candidate (its values, then a
-            // 16-byte head: key, then origin and row), slot CL the row at the pivot position (from
-            // CTA 0). Rows are below 2^32 (n <= kPanelRows), so origin and row take 32 bits each.
-            // Senders write it with st.async; inbox_bar[parity] counts the bytes.
-            __shared__ __align__(16) T inbox[2][kClusterCtas + 1][W];
-            __shared__ __align__(16) unsigned long long inbox_head[2][kClusterCtas + 1][2];
+            // By column parity: each warp's candidate, and the inbox, whose slot q holds CTA q's
+            // candidate. Senders write the inbox with st.async; inbox_bar[parity] counts the bytes.
+            __shared__ Candidate<T> published[2][WARPS];
+            __shared__ Candidate<T> inbox[2][kClusterCtas];
             __shared__ __align__(8) unsigned long long inbox_bar[2];
             __shared__ bool stalled;
-            __shared__ __align__(16) T jbuf[2][W];  // CTA 0: the row at the pivot position
-            __shared__ unsigned long long jbuf_origin[2];
             __shared__ long long exchanges[W];  // CTA 0: piv[j0 + j]
             // CTA 0: U's rows of the panel (row j from column j0 + j on, at u_rows[j][0, width - j)) and
             // the positions they are stored at until the final permutation, written out at the end
@@ -268,70 +286,64 @@ namespace sci_cuda {
             chain_release();
             const unsigned c = cluster_rank(), t = threadIdx.x, lane = t % 32, warp = t / 32;
             const unsigned long long first = j0 + 1ull * c * kCtaRows;  // this CTA's first row
-            unsigned long long r[R], origin[R];
-            bool valid[R];
+            const unsigned last = static_cast<unsigned>(n - j0) - 1u;       // the panel's last row
+            int pos[R];  // the row's position now, from the panel's first row (-1: no row)
             unsigned mask[R];
             T v[R][W];  // at step j: v[i][p] = column j0 + j + p of row i
             const bool vector = width == W && (n * sizeof(T)) % 16 == 0;
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                r[i] = first + 1ull * i * TH + t;
-                valid[i] = r[i] < n;
-                origin[i] = r[i];
+                const unsigned long long row = first + 1ull * i * TH + t;
+                pos[i] = row < n ? static_cast<int>(row - j0) : -1;
                 mask[i] = 0;
-                if (valid[i] && vector) {
-                    load_row(a + r[i] * n + j0, v[i]);
+                if (pos[i] >= 0 && vector) {
+                    load_row(a + row * n + j0, v[i]);
                 } else {
 #pragma unroll
-                    for (int k = 0; k < W; ++k) v[i][k] = (valid[i] && k < width) ? a[r[i] * n + j0 + k] : T(0);
+                    for (int k = 0; k < W; ++k) v[i][k] = (pos[i] >= 0 && k < width) ? a[row * n + j0 + k] : T(0);
                 }
             }
 
-            // The warp's candidate for the column whose values sit at v[i][O], among rows `from` on: the
-            // best key and row, published by lane 0 at `parity`; returns the row (kNoRow: none). A NaN
-            // only stands at the pivot position itself, where the reference's comparisons against it
-            // all fail (decompose.hpp:35-38).
-            auto search = [&](auto offset, const int parity, const unsigned long long from) -> unsigned {
+            // The warp's candidate for the column whose values sit at v[i][O], among positions `from`
+            // on: its key and position, published at `parity` by the lane that holds it. That lane
+            // gets the position, every other -1. A NaN only stands at the pivot position itself, where
+            // the reference's comparisons against it all fail (decompose.hpp:35-38).
+            auto search = [&](auto offset, const int parity, const int from) -> int {
                 constexpr int O = decltype(offset)::value;
                 Key key = 0;
                 unsigned rel = kNoRow;
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
-                    if (valid[i] && r[i] >= from) {
+                    if (pos[i] >= from) {
                         const T m = fabs(v[i][O]);
-                        const bool candidate = m == m || r[i] == from;
+                        const bool candidate = m == m || pos[i] == from;
                         const Key k = candidate ? magnitude_key(m == m ? m : T(INFINITY)) : Key(0);
-                        const unsigned at = static_cast<unsigned>(r[i] - j0);
+                        const unsigned at = static_cast<unsigned>(pos[i]);
                         if (k > key || (k == key && k != 0 && at < rel)) {
                             key = k;
                             rel = at;
                         }
                     }
                 }
-                best_of_warp(key, rel);
-                if (lane == 0) {
-                    warp_key[parity][warp] = key;
-                    warp_rel[parity][warp] = rel;
+                const bool best = lane == best_of_warp(key, rel);
+                if (best) {
+                    published[parity][warp].key = key;
+                    published[parity][warp].at = rel;
                 }
-                return rel;
+                return best ? static_cast<int>(rel) : -1;  // no candidate: kNoRow, -1 too
             };
-            // The winning lane's values from v[i][O] on (Q of them, zero past the row's W) and origin at
-            // `parity`; in CTA 0 the thread holding row `from` (the next pivot position) stages it too.
-            auto stage_candidate = [&](auto offset, auto span, const int parity, const unsigned rel,
-                                       const unsigned long long from) {
+            // The candidate's values from v[i][O] on (Q of them, zero past the row's W) and its origin
+            // at `parity`, by the lane that holds it.
+            auto stage_candidate = [&](auto offset, auto span, const int parity, const int at) {
                 constexpr int O = decltype(offset)::value, Q = decltype(span)::value;
+                if (at < 0) return;
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
-                    if (rel != kNoRow && r[i] - j0 == rel) {
+                    if (pos[i] == at) {
 #pragma unroll
-                        for (int k = 0; k < Q; ++k) warp_values[parity][warp][k] = k + O < W ? v[i][k + O] : T(0);
-                        warp_origin[parity][warp] = origin[i];
+                        for (int k = 0; k < Q; ++k) published[parity][warp].values[k] = k + O < W ? v[i][k + O] : T(0);
+                        published[parity][warp].origin = c * kCtaRows + i * TH + t;
                     }
-                }
-                if (c == 0 && t == static_cast<unsigned>(from - j0)) {  // row `from` is row 0 of that thread
-#pragma unroll
-                    for (int k = 0; k < Q; ++k) jbuf[parity][k] = k + O < W ? v[0][k + O] : T(0);
-                    jbuf_origin[parity] = origin[0];
                 }
             };
 
@@ -341,39 +353,26 @@ namespace sci_cuda {
             auto column = [&](auto span, const int j) {
                 constexpr int Q = decltype(span)::value;
                 const int par = j & 1;
-                const unsigned long long row_j = j0 + j;
-                __syncthreads();  // every warp's candidate (and CTA 0's pivot-position row) is staged
-                // 1. warp 0: the CTA's candidate; lane q sends it to CTA q (and lane q of CTA 0's warp 1
-                //    the pivot-position row), 16 bytes per store, the message's words read from shared
-                //    memory before the first store. A slot of parity par is rewritten two columns later, after every
-                //    reader has taken its pivot from it (each CTA's next message follows its own
-                //    barrier of the column in between, which its warps reach only after reading).
-                constexpr unsigned kValueBytes = Q * sizeof(T), kMessage = kValueBytes + 16;
-                static_assert(kValueBytes % 16 == 0, "16-byte stores");
-                // One message: the values, then a 16-byte head (key; origin and row, 32 bits each).
-                auto send = [&](const T *values, unsigned slot, unsigned long long k, unsigned long long o, unsigned rw) {
-                    const unsigned bar = remote(&inbox_bar[par], lane);
-                    uint4 words[kValueBytes / 16];
+                __syncthreads();  // every warp's candidate is staged
+                // 1. the CTA's candidate, by each of the first warps for its share of the CTAs: one
+                //    store sends a whole message, 16 bytes per lane, values then head. A slot of
+                //    parity par is rewritten two columns later, after every reader has taken its
+                //    pivot from it (each CTA's next message follows its own barrier of the column in
+                //    between, which its warps reach only after reading).
+                constexpr unsigned kWords = Q * sizeof(T) / 16, kHead = sizeof(T) * W / 16;
+                static_assert(Q * sizeof(T) % 16 == 0, "16-byte stores");
+                if (warp < SENDERS) {
+                    Key k2 = lane < WARPS ? static_cast<Key>(published[par][lane].key) : Key(0);
+                    const unsigned source = best_of_warp(k2, lane < WARPS ? published[par][lane].at : kNoRow);
+                    if (lane <= kWords) {
+                        const unsigned word = lane < kWords ? lane : kHead;
+                        const uint4 x = reinterpret_cast<const uint4 *>(&published[par][source])[word];
 #pragma unroll
-                    for (unsigned m = 0; m < kValueBytes / 16; ++m) words[m] = reinterpret_cast<const uint4 *>(values)[m];
-                    const unsigned base = remote(&inbox[par][slot][0], lane);
-                    const unsigned head = remote(&inbox_head[par][slot][0], lane);
-#pragma unroll
-                    for (unsigned m = 0; m < kValueBytes / 16; ++m)
-                        send16(base + 16 * m, words[m].x, words[m].y, words[m].z, words[m].w, bar);
-                    send16(head, static_cast<unsigned>(k), static_cast<unsigned>(k >> 32), static_cast<unsigned>(o), rw, bar);
-                };
-                if (warp == 0) {
-                    Key k2 = lane < WARPS ? warp_key[par][lane] : Key(0);
-                    unsigned r2 = lane < WARPS ? warp_rel[par][lane] : kNoRow;
-                    best_of_warp(k2, r2);
-                    const unsigned source = r2 == kNoRow ? 0u : ((r2 - c * kCtaRows) % TH) / 32;
-                    if (lane < static_cast<unsigned>(kClusterCtas))
-                        send(warp_values[par][source], c, static_cast<unsigned long long>(k2), warp_origin[par][source], r2);
-                    if (lane == 0) barrier_expect(&inbox_bar[par], (kClusterCtas + 1) * kMessage);
-                } else if (warp == 1 && c == 0 && lane < static_cast<unsigned>(kClusterCtas)) {
-                    // CTA 0's pivot-position row, from another warp (another scheduler) at the same time
-                    send(jbuf[par], kClusterCtas, 0ull, jbuf_origin[par], 0u);
+                        for (unsigned to = 0; to < kClusterCtas; to += SENDERS)
+                            send16(remote(reinterpret_cast<uint4 *>(&inbox[par][c]) + word, to + warp), x.x, x.y, x.z, x.w,
+                                   remote(&inbox_bar[par], to + warp));
+                    }
+                    if (warp == 0 && lane == 0) barrier_expect(&inbox_bar[par], kClusterCtas * (kWords + 1) * 16);
                 }
                 // 2. every warp waits for its CTA's inbox to fill (a bounded wait: one that runs out
                 //    flags the status, and no later column waits) and takes the pivot from it
@@ -384,46 +383,37 @@ namespace sci_cuda {
                 __syncwarp();
                 Key k3 = 0;
                 unsigned r3 = kNoRow;
-                unsigned long long org = 0;
                 if (lane < kClusterCtas) {
-                    k3 = static_cast<Key>(inbox_head[par][lane][0]);
-                    const unsigned long long where = inbox_head[par][lane][1];
-                    org = where & 0xFFFFFFFFull;
-                    r3 = static_cast<unsigned>(where >> 32);
+                    k3 = static_cast<Key>(inbox[par][lane].key);
+                    r3 = inbox[par][lane].at;
                 }
-                best_of_warp(k3, r3);
-                // the winner's CTA owns its row; no candidate cannot happen (row_j is one)
-                const unsigned q = r3 == kNoRow ? 0u : r3 / kCtaRows;
-                org = __shfl_sync(0xffffffffu, org, q);
-                const unsigned long long prow = r3 == kNoRow ? row_j : j0 + r3;
-                const T *const pivot_row = inbox[par][q];
-                if (c == 0 && t == 0) exchanges[j] = static_cast<long long>(prow);
-                constexpr int E = 16 / sizeof(T);  // pivot-row values per 16-byte load
+                // the CTA whose candidate wins (no candidate cannot happen: the pivot position is one)
+                const unsigned q = best_of_warp(k3, r3);
+                const T *const pivot_row = inbox[par][q].values;
                 const T diagonal = pivot_row[0];
+                // the pivot's position; the bound holds an inbox that did not fill (kStatusTimeout) to
+                // the panel's rows, so that no later store leaves the matrix
+                const int pivot = static_cast<int>(min(inbox[par][q].at, last));
+                if (c == 0 && warp == WARPS - 1) {
+                    // U's row j0 + j from column j0 + j on, kept for the end
+                    if (lane < Q) u_rows[j][lane] = pivot_row[lane];
+                    if (lane == 0) {
+                        u_origin[j] = j0 + min(inbox[par][q].origin, last);
+                        exchanges[j] = static_cast<long long>(j0) + pivot;
+                    }
+                }
                 T l[R];
                 bool below[R];
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
-                    if (r[i] == prow && prow != row_j) {
-                        // this row moves to the pivot's old place: it takes the displaced row's values
-#pragma unroll
-                        for (int k = 0; k < Q; k += E) load16(&inbox[par][kClusterCtas][k], &v[i][k]);
-                        origin[i] = inbox_head[par][kClusterCtas][1] & 0xFFFFFFFFull;
-                    }
-                    if (r[i] == row_j) {
-                        // the pivot row is final: U's row j0 + j from column j0 + j on, kept for the end
-                        // (16-byte shared stores here instead of Q scalar global stores in the
-                        // column's critical warp)
-#pragma unroll
-                        for (int k = 0; k < Q; k += E)
-                            *reinterpret_cast<uint4 *>(&u_rows[j][k]) = *reinterpret_cast<const uint4 *>(pivot_row + k);
-                        origin[i] = org;
-                        u_origin[j] = org;
-                    }
+                    // the exchange: the pivot row takes position j and the row there the pivot's; the
+                    // values stay where they are
+                    const int from = pos[i];
+                    pos[i] = from == j ? pivot : (from == pivot ? j : from);
                     // 3. eliminate below the pivot: l = a / pivot; a[k] -= l * pivot_row[k]; a zero
                     //    pivot leaves the column as it is (decompose.hpp:44-45). The next column
                     //    (v[i][1]) first.
-                    below[i] = valid[i] && r[i] > row_j;
+                    below[i] = pos[i] > j;
                     l[i] = v[i][0];
                     if (below[i] && diagonal != T(0)) {
                         l[i] = div(v[i][0], diagonal);
@@ -432,21 +422,16 @@ namespace sci_cuda {
                 }
                 // 4. the next column's search, while the rest of the elimination runs
                 const bool more = j + 1 < width;
-                const unsigned next_rel = more ? search(Span<1>{}, par ^ 1, row_j + 1) : kNoRow;
+                const int next = more ? search(Span<1>{}, par ^ 1, j + 1) : -1;
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
                     if (below[i] && diagonal != T(0)) eliminate_tail<Q>(v[i], l[i], pivot_row);
                     if (below[i]) {
-                        v[i][0] = l[i];
-                        if (origin[i] == r[i]) {
-                            stage[j * P + static_cast<int>(r[i] - first)] = l[i];
-                            mask[i] |= 1u << j;
-                        } else {
-                            a[origin[i] * n + row_j] = l[i];
-                        }
+                        stage[j * P + i * TH + static_cast<int>(t)] = l[i];
+                        mask[i] |= 1u << j;
                     }
                 }
-                if (more) stage_candidate(Span<1>{}, span, par ^ 1, next_rel, row_j + 1);
+                if (more) stage_candidate(Span<1>{}, span, par ^ 1, next);
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
 #pragma unroll
@@ -461,7 +446,7 @@ namespace sci_cuda {
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             }
             // column 0's candidates
-            stage_candidate(Span<0>{}, Span<W>{}, 0, search(Span<0>{}, 0, j0), j0);
+            stage_candidate(Span<0>{}, Span<W>{}, 0, search(Span<0>{}, 0, 0));
             cluster_sync();  // every CTA's inbox barriers exist before the first message
 #pragma unroll 1
             for (int j = 0; j < width; ++j) {
@@ -475,7 +460,7 @@ namespace sci_cuda {
             // position the row started in; move the rows the exchanges displaced: all reads, a
             // cluster barrier, then all writes.
 #pragma unroll
-            for (int i = 0; i < R; ++i) home[r[i] - first] = mask[i];
+            for (int i = 0; i < R; ++i) home[i * TH + t] = mask[i];
             __syncthreads();
             for (int row = warp; row < kCtaRows; row += WARPS) {
                 const unsigned long long g = first + row;
@@ -491,18 +476,20 @@ namespace sci_cuda {
             cluster_sync();
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                if (valid[i] && origin[i] != r[i]) {
+                const unsigned long long row = first + 1ull * i * TH + t;
+                if (pos[i] >= 0 && j0 + pos[i] != row) {
 #pragma unroll
-                    for (int k = 0; k < W; ++k) v[i][k] = k < width ? a[origin[i] * n + j0 + k] : T(0);
+                    for (int k = 0; k < W; ++k) v[i][k] = k < width ? a[row * n + j0 + k] : T(0);
                 }
             }
             cluster_sync();  // also: no CTA leaves while another may still read its shared memory
 #pragma unroll
             for (int i = 0; i < R; ++i) {
-                if (valid[i] && origin[i] != r[i]) {
+                const unsigned long long row = first + 1ull * i * TH + t;
+                if (pos[i] >= 0 && j0 + pos[i] != row) {
 #pragma unroll
                     for (int k = 0; k < W; ++k)
-                        if (k < width) a[r[i] * n + j0 + k] = v[i][k];
+                        if (k < width) a[(j0 + pos[i]) * n + j0 + k] = v[i][k];
                 }
             }
             if (c == 0 && warp == 0) {
