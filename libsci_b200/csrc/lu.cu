@@ -81,7 +81,7 @@ namespace sci_cuda {
         }
 
         // The panel's net row movement: after its exchanges, row rows[i] holds what row src[i] held.
-        // Only rows the panel touched appear (at most twice its width).
+        // Only rows the panel touched appear (at most twice its width), in no order.
         struct Movement {
             long long count;
             long long rows[64];
@@ -132,12 +132,12 @@ namespace sci_cuda {
             return static_cast<unsigned>(__ffs(holders)) - 1u;
         }
         // A candidate for the pivot: its row's values from the current column on, and the head that the
-        // choice is made by. Rows are below 2^32 (n <= kPanelRows), so origin and position take 32
-        // bits each. The values of one row and the head are 9 16-byte words.
+        // choice is made by. Rows are below 2^32 (n <= kPanelRows), so a position takes 32 bits.
+        // The values of one row and the head are 9 16-byte words.
         template <typename T> struct alignas(16) Candidate {
             T values[PanelWidth<T>::value];
             unsigned long long key;
-            unsigned origin, at;  // from the panel's first row: where the row started, where it is now
+            unsigned at, unused;  // the row's position, from the panel's first row
         };
         template <int N> struct Span {
             static constexpr int value = N;
@@ -235,10 +235,9 @@ namespace sci_cuda {
         // the current column is always v[i][0] (the column loop stays rolled: unrolled, every column
         // ran cold out of the instruction cache).
         //
-        // An exchange moves no values: a row stays in its thread (its origin) and only its position
-        // changes, in the two threads concerned. A row's multipliers of L are staged in shared memory
-        // and written out coalesced at the end, as are the pivot rows of U, at the rows' origins; a
-        // final permutation moves the at most 2 W displaced rows to their positions.
+        // An exchange moves no values: a row stays in its thread and only its position changes, in the
+        // two threads concerned. A row's multipliers of L are staged in shared memory and written out
+        // coalesced at the end, as are the pivot rows of U, each row at the position it ends at.
         //
         // Per column: each warp's best row is published in shared memory; after one CTA barrier, up to
         // four warps (one per scheduler) each reduce the warps' candidates and send the winner to
@@ -256,8 +255,10 @@ namespace sci_cuda {
         // order 8192 (8192 columns in 256 panels): 20.0 ms when an exchange moved the rows' values (a
         // second message from CTA 0 and scattered stores of the moved rows' multipliers), 19.2 ms with
         // rows kept in place, 18.8 ms with a message sent by one store whose lanes hold its 16-byte
-        // words (one lane sent all of a CTA's words before). 8 and 16 sending warps: 18.8 ms each;
-        // CTAs of 256 threads with two rows a thread: 7% slower.
+        // words (one lane sent all of a CTA's words before), 18.0 ms with every row written once, at
+        // the position it ends at, and its movement recorded by its own thread (before: written where
+        // it started, read back and moved, while one warp replayed the exchanges for the movement). 8
+        // and 16 sending warps: no change; CTAs of 256 threads with two rows a thread: 7% slower.
         template <typename T, int CL, int ROWS>
         __global__ void __launch_bounds__(kPanelBlock, 1)
                 panel_factor(T *a, unsigned long long n, unsigned long long j0, int width, long long *piv, Movement *moved,
@@ -269,6 +270,7 @@ namespace sci_cuda {
             extern __shared__ __align__(16) unsigned char panel_shared[];
             T *stage = reinterpret_cast<T *>(panel_shared);  // stage[k * P + local row]
             __shared__ unsigned home[kCtaRows];          // bit k: stage holds column k of the row
+            __shared__ int place[kCtaRows];              // the position the row ends at
             using Key = typename MagnitudeKey<T>::type;
             // By column parity: each warp's candidate, and the inbox, whose slot q holds CTA q's
             // candidate. Senders write the inbox with st.async; inbox_bar[parity] counts the bytes.
@@ -277,10 +279,9 @@ namespace sci_cuda {
             __shared__ __align__(8) unsigned long long inbox_bar[2];
             __shared__ bool stalled;
             __shared__ long long exchanges[W];  // CTA 0: piv[j0 + j]
-            // CTA 0: U's rows of the panel (row j from column j0 + j on, at u_rows[j][0, width - j)) and
-            // the positions they are stored at until the final permutation, written out at the end
+            // CTA 0: U's rows of the panel (row j from column j0 + j on, at u_rows[j][0, width - j)),
+            // written out at the end
             __shared__ __align__(16) T u_rows[W][W];
-            __shared__ unsigned long long u_origin[W];
 
             chain_wait();
             chain_release();
@@ -332,8 +333,8 @@ namespace sci_cuda {
                 }
                 return best ? static_cast<int>(rel) : -1;  // no candidate: kNoRow, -1 too
             };
-            // The candidate's values from v[i][O] on (Q of them, zero past the row's W) and its origin
-            // at `parity`, by the lane that holds it.
+            // The candidate's values from v[i][O] on (Q of them, zero past the row's W) at
+            // `parity`, by the lane that holds it.
             auto stage_candidate = [&](auto offset, auto span, const int parity, const int at) {
                 constexpr int O = decltype(offset)::value, Q = decltype(span)::value;
                 if (at < 0) return;
@@ -342,7 +343,6 @@ namespace sci_cuda {
                     if (pos[i] == at) {
 #pragma unroll
                         for (int k = 0; k < Q; ++k) published[parity][warp].values[k] = k + O < W ? v[i][k + O] : T(0);
-                        published[parity][warp].origin = c * kCtaRows + i * TH + t;
                     }
                 }
             };
@@ -397,10 +397,7 @@ namespace sci_cuda {
                 if (c == 0 && warp == WARPS - 1) {
                     // U's row j0 + j from column j0 + j on, kept for the end
                     if (lane < Q) u_rows[j][lane] = pivot_row[lane];
-                    if (lane == 0) {
-                        u_origin[j] = j0 + min(inbox[par][q].origin, last);
-                        exchanges[j] = static_cast<long long>(j0) + pivot;
-                    }
+                    if (lane == 0) exchanges[j] = static_cast<long long>(j0) + pivot;
                 }
                 T l[R];
                 bool below[R];
@@ -456,92 +453,45 @@ namespace sci_cuda {
                 else if (live > W / 4) column(Span<W / 2>{}, j);
                 else column(Span<W / 4>{}, j);
             }
-            // The staged multipliers, one row per warp store. Then every row's panel values sit at the
-            // position the row started in; move the rows the exchanges displaced: all reads, a
-            // cluster barrier, then all writes.
+            // Every row was read at the start, so each goes straight to the position it ends at: the
+            // staged multipliers, one row per warp store, and (CTA 0) U's rows.
+            if (c == 0 && t == 0) {
+                atomicExch(reinterpret_cast<unsigned long long *>(&moved->count), 0ull);
+                __threadfence();
+            }
 #pragma unroll
-            for (int i = 0; i < R; ++i) home[i * TH + t] = mask[i];
+            for (int i = 0; i < R; ++i) {
+                home[i * TH + t] = mask[i];
+                place[i * TH + t] = pos[i];
+            }
             __syncthreads();
             for (int row = warp; row < kCtaRows; row += WARPS) {
-                const unsigned long long g = first + row;
-                if (g >= n) break;
-                if (lane < static_cast<unsigned>(width) && (home[row] >> lane & 1u)) a[g * n + j0 + lane] = stage[lane * P + row];
+                if (first + row >= n) break;
+                if (lane < static_cast<unsigned>(width) && (home[row] >> lane & 1u))
+                    a[(j0 + place[row]) * n + j0 + lane] = stage[lane * P + row];
             }
             if (c == 0) {
-                // U's rows, at the positions the pivot rows started in (moved with them below)
+                if (t < static_cast<unsigned>(width)) piv[j0 + t] = exchanges[t];
                 for (int j = warp; j < width; j += WARPS)
-                    if (lane < static_cast<unsigned>(width - j)) a[u_origin[j] * n + j0 + j + lane] = u_rows[j][lane];
+                    if (lane < static_cast<unsigned>(width - j)) a[(j0 + j) * n + j0 + j + lane] = u_rows[j][lane];
             }
-            __threadfence();
-            cluster_sync();
+            cluster_sync();  // the count is zero; and no CTA leaves while another may still write its shared memory
+            // The net movement of rows, in any order: a reader takes every row before it writes one. At
+            // most 2 W rows moved; the bound is for an inbox that did not fill.
+            constexpr unsigned long long kMoved = sizeof(moved->rows) / sizeof(moved->rows[0]);
 #pragma unroll
             for (int i = 0; i < R; ++i) {
                 const unsigned long long row = first + 1ull * i * TH + t;
                 if (pos[i] >= 0 && j0 + pos[i] != row) {
-#pragma unroll
-                    for (int k = 0; k < W; ++k) v[i][k] = k < width ? a[row * n + j0 + k] : T(0);
-                }
-            }
-            cluster_sync();  // also: no CTA leaves while another may still read its shared memory
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const unsigned long long row = first + 1ull * i * TH + t;
-                if (pos[i] >= 0 && j0 + pos[i] != row) {
-#pragma unroll
-                    for (int k = 0; k < W; ++k)
-                        if (k < width) a[(j0 + pos[i]) * n + j0 + k] = v[i][k];
-                }
-            }
-            if (c == 0 && warp == 0) {
-                // The net movement of rows: the exchanges applied in order to a table of the rows they
-                // touch (at most 2W), one warp, each lane holding two table entries.
-                __syncwarp();
-                long long row_a = lane < static_cast<unsigned>(width) ? static_cast<long long>(j0 + lane) : -1;
-                long long row_b = -1;
-                long long src_a = row_a, src_b = -1;
-                int count = width;
-                if (lane < static_cast<unsigned>(width)) piv[j0 + lane] = exchanges[lane];
-                for (int j = 0; j < width; ++j) {
-                    const long long p = exchanges[j];
-                    // where p sits in the table: entry index, or -1
-                    const unsigned in_a = __ballot_sync(0xffffffffu, row_a == p);
-                    const unsigned in_b = __ballot_sync(0xffffffffu, row_b == p);
-                    int at = in_a ? __ffs(in_a) - 1 : (in_b ? 32 + __ffs(in_b) - 1 : -1);
-                    if (at < 0) {
-                        at = count++;
-                        if (at < 32) {
-                            if (lane == static_cast<unsigned>(at)) row_a = src_a = p;
-                        } else if (lane == static_cast<unsigned>(at - 32)) {
-                            row_b = src_b = p;
-                        }
-                    }
-                    // exchange the contents of entries j and at
-                    const long long from_j = __shfl_sync(0xffffffffu, src_a, j);
-                    const long long from_at = at < 32 ? __shfl_sync(0xffffffffu, src_a, at & 31)
-                                                      : __shfl_sync(0xffffffffu, src_b, at & 31);
-                    if (lane == static_cast<unsigned>(j)) src_a = from_at;
-                    if (at < 32) {
-                        if (lane == static_cast<unsigned>(at)) src_a = from_j;
-                    } else if (lane == static_cast<unsigned>(at - 32)) {
-                        src_b = from_j;
+                    unsigned long long *const count = reinterpret_cast<unsigned long long *>(&moved->count);
+                    const unsigned long long slot = atomicAdd(count, 1ull);
+                    if (slot < kMoved) {
+                        moved->rows[slot] = static_cast<long long>(j0) + pos[i];
+                        moved->src[slot] = static_cast<long long>(row);
+                    } else {
+                        atomicMin(count, kMoved);
                     }
                 }
-                // keep the entries that moved, in order
-                const bool keep_a = static_cast<int>(lane) < count && row_a != src_a;
-                const bool keep_b = static_cast<int>(lane) + 32 < count && row_b != src_b;
-                const unsigned mask_a = __ballot_sync(0xffffffffu, keep_a), mask_b = __ballot_sync(0xffffffffu, keep_b);
-                const unsigned below = (1u << lane) - 1u;
-                if (keep_a) {
-                    const int slot = __popc(mask_a & below);
-                    moved->rows[slot] = row_a;
-                    moved->src[slot] = src_a;
-                }
-                if (keep_b) {
-                    const int slot = __popc(mask_a) + __popc(mask_b & below);
-                    moved->rows[slot] = row_b;
-                    moved->src[slot] = src_b;
-                }
-                if (lane == 0) moved->count = __popc(mask_a) + __popc(mask_b);
             }
         }
 
