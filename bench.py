@@ -808,8 +808,8 @@ def run_batch(args) -> dict:
 
 def run_solves(args) -> dict:
     """Batching of solves: 4096 independent systems, n ~ U[8, 256] (seeded), A = G + n I (G ~ N(0,1)),
-    one right-hand side ~ N(0,1), FP32 LU + FP64 refinement, one graph replay (block size tuned per
-    order bucket). Beside it: a loop of single sci_cuda_solve calls (the plain form, sampled) and
+    one right-hand side ~ N(0,1), FP32 LU + FP64 refinement, one graph replay (one launch per
+    order group). Beside it: a loop of single sci_cuda_solve calls (the plain form, sampled) and
     libsci's CPU solve<double> per system (sampled)."""
     import torch
 

@@ -77,9 +77,9 @@ namespace sci_cuda {
         std::string name;
 
         ReduceState *state{nullptr};   // reduction scratch (device)
-        double *result{nullptr};       // reduction result (device), with the status word 8 bytes on
+        double *result{nullptr};       // device: a spare double, with the status word 8 bytes on
         int *status{nullptr};          // device-side error word (in result's allocation)
-        double *host_result{nullptr};  // pinned, with host_status 8 bytes on: one copy reads both
+        double *host_result{nullptr};  // pinned, with host_status 8 bytes on: blocking reductions write both
         int *host_status{nullptr};     // pinned (in host_result's allocation)
         unsigned *notice_word{nullptr};  // pinned (in host_result's allocation): the last reduction's notice
         unsigned notice_value{0};
