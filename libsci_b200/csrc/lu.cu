@@ -361,39 +361,47 @@ namespace sci_cuda {
                 //    between, which its warps reach only after reading).
                 constexpr unsigned kWords = Q * sizeof(T) / 16, kHead = sizeof(T) * W / 16;
                 static_assert(Q * sizeof(T) % 16 == 0, "16-byte stores");
-                if (warp < SENDERS) {
+                const Candidate<T> *winner;
+                if constexpr (CL == 1) {
+                    // one CTA: every warp takes the pivot from the warps' candidates themselves, which
+                    // are written again only after the next column's barrier
                     Key k2 = lane < WARPS ? static_cast<Key>(published[par][lane].key) : Key(0);
-                    const unsigned source = best_of_warp(k2, lane < WARPS ? published[par][lane].at : kNoRow);
-                    if (lane <= kWords) {
-                        const unsigned word = lane < kWords ? lane : kHead;
-                        const uint4 x = reinterpret_cast<const uint4 *>(&published[par][source])[word];
-#pragma unroll
-                        for (unsigned to = 0; to < kClusterCtas; to += SENDERS)
-                            send16(remote(reinterpret_cast<uint4 *>(&inbox[par][c]) + word, to + warp), x.x, x.y, x.z, x.w,
-                                   remote(&inbox_bar[par], to + warp));
+                    winner = &published[par][best_of_warp(k2, lane < WARPS ? published[par][lane].at : kNoRow)];
+                } else {
+                    if (warp < SENDERS) {
+                        Key k2 = lane < WARPS ? static_cast<Key>(published[par][lane].key) : Key(0);
+                        const unsigned source = best_of_warp(k2, lane < WARPS ? published[par][lane].at : kNoRow);
+                        if (lane <= kWords) {
+                            const unsigned word = lane < kWords ? lane : kHead;
+                            const uint4 x = reinterpret_cast<const uint4 *>(&published[par][source])[word];
+    #pragma unroll
+                            for (unsigned to = 0; to < kClusterCtas; to += SENDERS)
+                                send16(remote(reinterpret_cast<uint4 *>(&inbox[par][c]) + word, to + warp), x.x, x.y, x.z, x.w,
+                                       remote(&inbox_bar[par], to + warp));
+                        }
+                        if (warp == 0 && lane == 0) barrier_expect(&inbox_bar[par], kClusterCtas * (kWords + 1) * 16);
                     }
-                    if (warp == 0 && lane == 0) barrier_expect(&inbox_bar[par], kClusterCtas * (kWords + 1) * 16);
+                    // 2. every warp waits for its CTA's inbox to fill (a bounded wait: one that runs out
+                    //    flags the status, and no later column waits) and takes the pivot from it
+                    if (!stalled && !barrier_wait(&inbox_bar[par], static_cast<unsigned>(j >> 1) & 1u) && lane == 0) {
+                        stalled = true;
+                        atomicOr(status, kStatusTimeout);
+                    }
+                    __syncwarp();
+                    Key k3 = 0;
+                    unsigned r3 = kNoRow;
+                    if (lane < kClusterCtas) {
+                        k3 = static_cast<Key>(inbox[par][lane].key);
+                        r3 = inbox[par][lane].at;
+                    }
+                    // the CTA whose candidate wins (no candidate cannot happen: the pivot position is one)
+                    winner = &inbox[par][best_of_warp(k3, r3)];
                 }
-                // 2. every warp waits for its CTA's inbox to fill (a bounded wait: one that runs out
-                //    flags the status, and no later column waits) and takes the pivot from it
-                if (!stalled && !barrier_wait(&inbox_bar[par], static_cast<unsigned>(j >> 1) & 1u) && lane == 0) {
-                    stalled = true;
-                    atomicOr(status, kStatusTimeout);
-                }
-                __syncwarp();
-                Key k3 = 0;
-                unsigned r3 = kNoRow;
-                if (lane < kClusterCtas) {
-                    k3 = static_cast<Key>(inbox[par][lane].key);
-                    r3 = inbox[par][lane].at;
-                }
-                // the CTA whose candidate wins (no candidate cannot happen: the pivot position is one)
-                const unsigned q = best_of_warp(k3, r3);
-                const T *const pivot_row = inbox[par][q].values;
+                const T *const pivot_row = winner->values;
                 const T diagonal = pivot_row[0];
                 // the pivot's position; the bound holds an inbox that did not fill (kStatusTimeout) to
                 // the panel's rows, so that no later store leaves the matrix
-                const int pivot = static_cast<int>(min(inbox[par][q].at, last));
+                const int pivot = static_cast<int>(min(winner->at, last));
                 if (c == 0 && warp == WARPS - 1) {
                     // U's row j0 + j from column j0 + j on, kept for the end
                     if (lane < Q) u_rows[j][lane] = pivot_row[lane];
