@@ -354,27 +354,28 @@ namespace sci_cuda {
                 constexpr int Q = decltype(span)::value;
                 const int par = j & 1;
                 __syncthreads();  // every warp's candidate is staged
-                // 1. the CTA's candidate, by each of the first warps for its share of the CTAs: one
-                //    store sends a whole message, 16 bytes per lane, values then head. A slot of
-                //    parity par is rewritten two columns later, after every reader has taken its
-                //    pivot from it (each CTA's next message follows its own barrier of the column in
-                //    between, which its warps reach only after reading).
                 constexpr unsigned kWords = Q * sizeof(T) / 16, kHead = sizeof(T) * W / 16;
                 static_assert(Q * sizeof(T) % 16 == 0, "16-byte stores");
                 const Candidate<T> *winner;
                 if constexpr (CL == 1) {
                     // one CTA: every warp takes the pivot from the warps' candidates themselves, which
-                    // are written again only after the next column's barrier
+                    // are written again only after the next column's barrier (through the inbox, as
+                    // below, a float solve of order 500 took 909 us instead of 798)
                     Key k2 = lane < WARPS ? static_cast<Key>(published[par][lane].key) : Key(0);
                     winner = &published[par][best_of_warp(k2, lane < WARPS ? published[par][lane].at : kNoRow)];
                 } else {
+                    // 1. the CTA's candidate, by each of the first warps for its share of the CTAs:
+                    //    one store sends a whole message, 16 bytes per lane, values then head. A slot
+                    //    of parity par is rewritten two columns later, after every reader has taken
+                    //    its pivot from it (each CTA's next message follows its own barrier of the
+                    //    column in between, which its warps reach only after reading).
                     if (warp < SENDERS) {
                         Key k2 = lane < WARPS ? static_cast<Key>(published[par][lane].key) : Key(0);
                         const unsigned source = best_of_warp(k2, lane < WARPS ? published[par][lane].at : kNoRow);
                         if (lane <= kWords) {
                             const unsigned word = lane < kWords ? lane : kHead;
                             const uint4 x = reinterpret_cast<const uint4 *>(&published[par][source])[word];
-    #pragma unroll
+#pragma unroll
                             for (unsigned to = 0; to < kClusterCtas; to += SENDERS)
                                 send16(remote(reinterpret_cast<uint4 *>(&inbox[par][c]) + word, to + warp), x.x, x.y, x.z, x.w,
                                        remote(&inbox_bar[par], to + warp));
