@@ -2556,7 +2556,10 @@ namespace {
         if (int code = ctx.drain()) return code;
         berr = 0.0;
         for (unsigned long long j = 0; j < width; ++j) {
-            const double e = host[j] / (*a_norm * host[width + j] + b_norm[j]);
+            // zero over zero: a right-hand side of zeros with its exact solution, not a NaN that would end the
+            // refinement of the other columns
+            const double scale = *a_norm * host[width + j] + b_norm[j];
+            const double e = host[j] == 0.0 && scale == 0.0 ? 0.0 : host[j] / scale;
             berr = (e > berr || e != e) ? e : berr;
         }
         return SCI_CUDA_OK;

@@ -24,7 +24,7 @@
 //    for the substitutions.
 // Refinement: x = 0, r = b; repeat { d = U^-1 L^-1 P r in FP32; x += d; r = b - A x in FP64 } until the
 // normwise backward error |r|_inf / (|A|_inf |x|_inf + |b|_inf) is at most `target` or stops halving
-// (at most 30 corrections): the rule of sci_cuda_solve's refinement. A substitution step is a 32 x 32
+// (at most 30 corrections): the rule of sci_cuda_solve's refinement (a column of zeros counts as solved). A substitution step is a 32 x 32
 // product with the block's inverse by one warp and an update of the other rows from their own L or U.
 //
 // What bounds it: the chain of columns (700 cycles each at order 128, 790 at 256: two barriers, a
@@ -906,7 +906,11 @@ namespace sci_cuda {
             for (int q = 0; q < NR; ++q) {
                 double rm = 0.0, xm = 0.0;
                 for (int v = 0; v < warps; ++v) rm = small_larger(maxima[v][q], rm), xm = small_larger(maxima[v][NR + q], xm);
-                if (q < static_cast<int>(sys.columns)) berr = small_larger(rm / (a_norm * xm + b_norm[q]), berr);
+                // zero over zero: a right-hand side of zeros with its exact solution, not a NaN that would end
+                // the refinement of the other columns
+                const double scale = a_norm * xm + b_norm[q];
+                const double error = rm == 0.0 && scale == 0.0 ? 0.0 : rm / scale;
+                if (q < static_cast<int>(sys.columns)) berr = small_larger(error, berr);
             }
             ++count;
             if (count >= 30 || !(berr > target) || !(berr < 0.5 * previous)) break;
