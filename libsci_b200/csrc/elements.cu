@@ -405,7 +405,8 @@ namespace sci_cuda {
             if (slot_file() > 48 * 1024) threads = 128;
             while (threads > 64 && slot_file() > ctx.shared_limit) threads /= 2;
             const size_t smem = slot_file();
-            if (smem > 48 * 1024) {
+            // with the kernel's own shared memory (less than a kilobyte) past what a launch gets unasked
+            if (smem + 1024 > 48 * 1024) {
                 if (smem > ctx.shared_limit) return ctx.fail(SCI_CUDA_ERROR_INVALID, "%u temporaries exceed shared memory", chunk.temporaries);
                 if (int code = ctx.check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                               static_cast<int>(smem)),
