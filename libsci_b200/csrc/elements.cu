@@ -415,7 +415,9 @@ namespace sci_cuda {
             }
             const unsigned long long tile = 1ull * lanes * threads;
             const unsigned long long tiles = (count + tile - 1) / tile;
-            const unsigned long long most = 1ull * ctx.sms * ctx.blocks_per_sm(kernel, threads, smem);
+            // a reduction's blocks leave a partial each in the context's state, which holds kMaxBlocks of them
+            unsigned long long most = 1ull * ctx.sms * ctx.blocks_per_sm(kernel, threads, smem);
+            if (reducing && most > kMaxBlocks) most = kMaxBlocks;
             const unsigned grid = static_cast<unsigned>(tiles < most ? tiles : most);
             if (reducing) L.notice = ctx.next_notice();
             void *args[] = {&L};
