@@ -145,7 +145,7 @@ namespace sci_cuda {
         constexpr int kWarps = kSmallMax / 32;
         constexpr unsigned kAll = 0xffffffffu;
         __shared__ __align__(16) float pivot_rows[2][32];      // the pivot's row of the block, by column parity
-        __shared__ __align__(8) float2 pivot_reciprocals[2];   // a scale and the scaled pivot's reciprocal
+        __shared__ __align__(16) float4 divisors[2];           // a scale, the scaled pivot's reciprocal, the scaled pivot
         __shared__ __align__(16) uint2 best[kWarps];           // each warp's largest key (0: no row left) and its place
         __shared__ __align__(16) float to_solve[32 * NR], solved[32 * NR];  // a substitution step's block, in and out
         __shared__ double maxima[kWarps][2 * NR];
@@ -347,12 +347,14 @@ namespace sci_cuda {
                     const unsigned own_place = static_cast<unsigned>(second ? spot[R - 1] : spot[0]);
                     const float own_value = second ? w[R - 1][0] : w[0][0];
                     const unsigned most = __reduce_max_sync(kAll, own_key);
-                    // 1 / value, of use if this row is the pivot's, by one step of Newton's iteration on the approximate
-                    // reciprocal; `scale` keeps that in range
+                    // 1 / value, of use if this row is the pivot's: a step of Newton's iteration on the approximate
+                    // reciprocal; `scale` keeps that and the quotients' remainders in range. An infinite pivot divides by 1
+                    // and multiplies by 0.
                     const float size = fabsf(own_value);
                     const float scale = size < 0x1p-96f ? 0x1p96f : (size > 0x1p96f ? 0x1p-96f : 1.0f);
                     const float scaled = own_value * scale, guess = __fdividef(1.0f, scaled);
-                    const float reciprocal = fmaf(guess, fmaf(-scaled, guess, 1.0f), guess);
+                    const bool infinite = size == INFINITY;
+                    const float reciprocal = infinite ? 0.0f : fmaf(guess, fmaf(-scaled, guess, 1.0f), guess);
                     unsigned mine = __ballot_sync(kAll, own_key == most);
                     if (mine & (mine - 1)) {  // equals: the lowest place
                         const unsigned lowest = __reduce_min_sync(kAll, own_key == most ? own_place : ~0u);
@@ -382,18 +384,23 @@ namespace sci_cuda {
 #pragma unroll
                         for (int v = 0; v < V; ++v) small_store_if(publishes, pivot + 4 * v, w[h][4 * v], w[h][4 * v + 1], w[h][4 * v + 2], w[h][4 * v + 3]);
                     }
-                    small_store_if(winner, &pivot_reciprocals[j & 1], __float_as_uint(scale), __float_as_uint(reciprocal));
+                    small_store_if(winner, &divisors[j & 1], scale, reciprocal, infinite ? 1.0f : scaled, 0.0f);
                     meet();
                     float4 u[V + 1];
                     u[V] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    const float2 inverse = pivot_reciprocals[j & 1];
+                    const float4 divisor = divisors[j & 1];
 #pragma unroll
                     for (int v = 0; v < V; ++v) u[v] = vector(pivot + 4 * v);
 #pragma unroll
                     for (int h = 0; h < R; ++h) {
                         const bool chosen = winner && second == (h > 0);
                         const bool act = live[h] && !chosen && u[0].x != 0.0f;
-                        const float quotient = w[h][0] * inverse.x * inverse.y;
+                        // The quotient from the reciprocal, corrected by its remainder (Markstein, Computation of elementary
+                        // functions on the IBM RISC System/6000, 1990): equal to the rounded division in 2^33 random
+                        // trials without denormal intermediates. The division itself waits for the pivot's row:
+                        // 291 us instead of 247 for 4096 systems of order 33 to 64 (238 uncorrected).
+                        const float dividend = w[h][0] * divisor.x, about = dividend * divisor.y;
+                        const float quotient = fmaf(fmaf(-about, divisor.z, dividend), divisor.y, about);
                         const float l = act ? quotient : 0.0f;  // a row that is done multiplies by zero
                         home(h, column, act ? quotient : w[h][0]);
                         spot[h] = chosen ? column : (spot[h] == column ? static_cast<int>(top.y) : spot[h]);
