@@ -10,8 +10,8 @@
 //
 // Factorisation, by 32-column blocks, left-looking: every earlier block K is applied to the block, and
 // the block is factored column by column.
-//  - applying block K: the 32 rows placed in it are published (shared memory); U_K = inv(L_KK) W_K is
-//    one small product by two warps; every row below subtracts L[row, K] U_K. A warp holds its 32
+//  - applying block K: the 32 rows placed in it are published (shared memory); U_K = L_KK^-1 W_K by
+//    substitution, a column per lane of one warp; every row below subtracts L[row, K] U_K. A warp holds its 32
 //    rows' entries of the block as tiles of 4 rows x 8 columns per lane through all K (a row per
 //    lane reads 33 values for 32 multiplications, and shared memory returns a quarter of what the
 //    multipliers consume: 6.3 thousand cycles a step at order 256; the tile reads 12 for 32), a pair of columns per FMA
@@ -20,12 +20,12 @@
 //    |value| (the lowest place among equals: the first row with the strictly largest |a|,
 //    include/linear/decompose.hpp:29-72; a zero pivot skips the column's elimination); after a barrier
 //    every warp knows the pivot, its thread publishes the row, and after another every thread eliminates.
-//  - the block's triangles are inverted in place (a warp each for L and U), for the products above and
-//    for the substitutions.
+// Inverses of the blocks' triangles in place of the substitutions, here and in the refinement, lost accuracy:
+// systems of order 48 and condition 1e6 took 4.9 corrections instead of 4.0.
 // Refinement: x = 0, r = b; repeat { d = U^-1 L^-1 P r in FP32; x += d; r = b - A x in FP64 } until the
 // normwise backward error |r|_inf / (|A|_inf |x|_inf + |b|_inf) is at most `target` or stops halving
-// (at most 30 corrections): the rule of sci_cuda_solve's refinement (a column of zeros counts as solved). A substitution step is a 32 x 32
-// product with the block's inverse by one warp and an update of the other rows from their own L or U.
+// (at most 30 corrections): the rule of sci_cuda_solve's refinement (a column of zeros counts as solved). A
+// substitution step is a block's triangle by one warp and an update of the other rows from their own L or U.
 //
 // What bounds it: the chain of columns (700 cycles each at order 128, 790 at 256: two barriers, a
 // warp-wide maximum and vote, four trips through shared memory) and of barriers; systems of order 152
@@ -62,7 +62,7 @@ namespace sci_cuda {
     inline unsigned long long small_shared_bytes(int most, int right_sides, int register_blocks) {
         unsigned long long bytes = 4ull * most * small_pitch(most, register_blocks);  // factors
         bytes += 2ull * 32 * kSmallPitch * 4;                    // published blocks (later: products with x)
-        bytes += 4ull * register_blocks * 32 * kSmallPitch;      // inverses of register blocks
+        bytes += 4ull * register_blocks * 32 * kSmallPitch;      // triangles of register blocks
         bytes += 8ull * most * right_sides;                      // x
         bytes += 2ull * 2 * most;                                // rows by position, positions by row
         return (bytes + 15) / 16 * 16;
@@ -97,6 +97,26 @@ namespace sci_cuda {
     }
 
     __device__ __forceinline__ double small_larger(double v, double m) { return (v > m || v != v) ? v : m; }  // NaN wins
+
+    // Division by a value that is known before the dividends: its reciprocal by a step of Newton's iteration on the approximate
+    // one, and the quotient corrected by its remainder (Markstein, Computation of elementary functions on the IBM RISC
+    // System/6000, 1990): equal to the rounded division in 2^33 random trials without denormal intermediates.
+    // `scale` keeps these in range; an infinite value divides by 1 and multiplies by 0. The division itself
+    // waits for the pivot's row: 291 us instead of 247 for 4096 systems of order 33 to 64 (238 uncorrected).
+    struct Divisor {
+        float scale, reciprocal, scaled;
+    };
+    __device__ __forceinline__ Divisor divisor_of(float value) {
+        const float size = fabsf(value);
+        const float scale = size < 0x1p-96f ? 0x1p96f : (size > 0x1p96f ? 0x1p-96f : 1.0f);
+        const float scaled = value * scale, guess = __fdividef(1.0f, scaled);
+        const bool infinite = size == INFINITY;
+        return Divisor{scale, infinite || size == 0.0f ? guess : fmaf(guess, fmaf(-scaled, guess, 1.0f), guess), infinite ? 1.0f : scaled};
+    }
+    __device__ __forceinline__ float quotient_of(float dividend, const Divisor &d) {
+        const float x = dividend * d.scale, about = x * d.reciprocal;
+        return fmaf(fmaf(-about, d.scaled, x), d.reciprocal, about);
+    }
 
     // Sums M values of every lane over the warp, M a power of two up to 8: lanes exchange halves of the
     // values while they can, so value m's sum ends in the lanes whose top bits spell m.
@@ -145,7 +165,7 @@ namespace sci_cuda {
         constexpr int kWarps = kSmallMax / 32;
         constexpr unsigned kAll = 0xffffffffu;
         __shared__ __align__(16) float pivot_rows[2][32];      // the pivot's row of the block, by column parity
-        __shared__ __align__(16) float4 divisors[2];           // a scale, the scaled pivot's reciprocal, the scaled pivot
+        __shared__ __align__(16) float4 divisors[2];           // the pivot as a Divisor
         __shared__ __align__(16) uint2 best[kWarps];           // each warp's largest key (0: no row left) and its place
         __shared__ __align__(16) float to_solve[32 * NR], solved[32 * NR];  // a substitution step's block, in and out
         __shared__ double maxima[kWarps][2 * NR];
@@ -163,10 +183,10 @@ namespace sci_cuda {
         float *A = reinterpret_cast<float *>(small_shared);
         unsigned char *cursor = small_shared + 4ull * n * P;
         float *published = reinterpret_cast<float *>(cursor);  // the block's rows as they were
-        float *u_block = published + 32 * kSmallPitch;         // and as rows of U (or a block's L and U to invert)
+        float *u_block = published + 32 * kSmallPitch;         // and as rows of U
         double *sums = reinterpret_cast<double *>(cursor);     // the rows' products with x, once the factors are done
         cursor += 2ull * 32 * kSmallPitch * 4;
-        float *inverses = reinterpret_cast<float *>(cursor);
+        float *triangles = reinterpret_cast<float *>(cursor);
         cursor += 4ull * RB * 32 * kSmallPitch;
         double *x = reinterpret_cast<double *>(cursor);
         unsigned short *rows = reinterpret_cast<unsigned short *>(x + n * NR);  // the row at each position
@@ -275,40 +295,31 @@ namespace sci_cuda {
 
         // ---- LU with partial pivoting
         int place = row ? tid : kSmallMax;
-        // row i of the inverse of block K's triangles (L's strictly below the diagonal, U's on and above it)
-        auto inverse_row = [&](int K, int i) -> float * {
-            if (RB > 0 && K >= SB) return inverses + ((K - SB) * 32 + i) * kSmallPitch;
+        // row i of block K's triangles: L's strictly below the diagonal, U's on and above it
+        auto triangle_row = [&](int K, int i) -> float * {
+            if (RB > 0 && K >= SB) return triangles + ((K - SB) * 32 + i) * kSmallPitch;
             return A + rows[32 * K + i] * P + 32 * K;
         };
-        // U_K = inv(L_KK) W_K: 64 threads, four rows and four columns each
-        auto product = [&](int K) {
-            if (tid < 64) {
-                const int i0 = (tid >> 3) * 4, c = (tid & 7) * 4;
-                float4 acc[4];
-                float *inverse[4];
+        // U_K = L_KK^-1 W_K by substitution, a column per lane of one warp
+        auto substitute = [&](int K) {
+            if (warp == 0) {
+                float v[32];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    acc[i] = vector(published + (i0 + i) * kSmallPitch + c);
-                    inverse[i] = inverse_row(K, i0 + i);
-                }
-                for (int k0 = 0; k0 <= (tid < 32 ? 12 : 28); k0 += 4) {
-                    float4 l[4];
+                for (int i = 0; i < 32; ++i) v[i] = published[i * kSmallPitch + lane];
+                static_for<32>([&](auto i_c) {
+                    constexpr int i = decltype(i_c)::value;
+                    float *l = triangle_row(K, i);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) l[i] = vector(inverse[i] + k0);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float4 v = vector(published + (k0 + e) * kSmallPitch + c);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float entry = e == 0 ? l[i].x : (e == 1 ? l[i].y : (e == 2 ? l[i].z : l[i].w));
-                            const float f = k0 + e < i0 + i ? entry : 0.0f;
-                            acc[i].x = fmaf(f, v.x, acc[i].x), acc[i].y = fmaf(f, v.y, acc[i].y);
-                            acc[i].z = fmaf(f, v.z, acc[i].z), acc[i].w = fmaf(f, v.w, acc[i].w);
-                        }
+                    for (int k = 0; k < i; k += 4) {
+                        const float4 q = vector(l + k);
+                        v[i] = fmaf(-q.x, v[k], v[i]);
+                        if (k + 1 < i) v[i] = fmaf(-q.y, v[k + 1], v[i]);
+                        if (k + 2 < i) v[i] = fmaf(-q.z, v[k + 2], v[i]);
+                        if (k + 3 < i) v[i] = fmaf(-q.w, v[k + 3], v[i]);
                     }
-                }
+                });
 #pragma unroll
-                for (int i = 0; i < 4; ++i) vector(u_block + (i0 + i) * kSmallPitch + c) = acc[i];
+                for (int i = 0; i < 32; ++i) u_block[i * kSmallPitch + lane] = v[i];
             }
         };
         // The columns of a block, R rows per thread of `crew` warps: w[h][0] is the next column, and the registers move
@@ -347,14 +358,7 @@ namespace sci_cuda {
                     const unsigned own_place = static_cast<unsigned>(second ? spot[R - 1] : spot[0]);
                     const float own_value = second ? w[R - 1][0] : w[0][0];
                     const unsigned most = __reduce_max_sync(kAll, own_key);
-                    // 1 / value, of use if this row is the pivot's: a step of Newton's iteration on the approximate
-                    // reciprocal; `scale` keeps that and the quotients' remainders in range. An infinite pivot divides by 1
-                    // and multiplies by 0.
-                    const float size = fabsf(own_value);
-                    const float scale = size < 0x1p-96f ? 0x1p96f : (size > 0x1p96f ? 0x1p-96f : 1.0f);
-                    const float scaled = own_value * scale, guess = __fdividef(1.0f, scaled);
-                    const bool infinite = size == INFINITY;
-                    const float reciprocal = infinite ? 0.0f : fmaf(guess, fmaf(-scaled, guess, 1.0f), guess);
+                    const Divisor own = divisor_of(own_value);  // of use if this row is the pivot's
                     unsigned mine = __ballot_sync(kAll, own_key == most);
                     if (mine & (mine - 1)) {  // equals: the lowest place
                         const unsigned lowest = __reduce_min_sync(kAll, own_key == most ? own_place : ~0u);
@@ -384,23 +388,19 @@ namespace sci_cuda {
 #pragma unroll
                         for (int v = 0; v < V; ++v) small_store_if(publishes, pivot + 4 * v, w[h][4 * v], w[h][4 * v + 1], w[h][4 * v + 2], w[h][4 * v + 3]);
                     }
-                    small_store_if(winner, &divisors[j & 1], scale, reciprocal, infinite ? 1.0f : scaled, 0.0f);
+                    small_store_if(winner, &divisors[j & 1], own.scale, own.reciprocal, own.scaled, 0.0f);
                     meet();
                     float4 u[V + 1];
                     u[V] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    const float4 divisor = divisors[j & 1];
+                    const float4 stored = divisors[j & 1];
+                    const Divisor divisor{stored.x, stored.y, stored.z};
 #pragma unroll
                     for (int v = 0; v < V; ++v) u[v] = vector(pivot + 4 * v);
 #pragma unroll
                     for (int h = 0; h < R; ++h) {
                         const bool chosen = winner && second == (h > 0);
                         const bool act = live[h] && !chosen && u[0].x != 0.0f;
-                        // The quotient from the reciprocal, corrected by its remainder (Markstein, Computation of elementary
-                        // functions on the IBM RISC System/6000, 1990): equal to the rounded division in 2^33 random
-                        // trials without denormal intermediates. The division itself waits for the pivot's row:
-                        // 291 us instead of 247 for 4096 systems of order 33 to 64 (238 uncorrected).
-                        const float dividend = w[h][0] * divisor.x, about = dividend * divisor.y;
-                        const float quotient = fmaf(fmaf(-about, divisor.z, dividend), divisor.y, about);
+                        const float quotient = quotient_of(w[h][0], divisor);
                         const float l = act ? quotient : 0.0f;  // a row that is done multiplies by zero
                         home(h, column, act ? quotient : w[h][0]);
                         spot[h] = chosen ? column : (spot[h] == column ? static_cast<int>(top.y) : spot[h]);
@@ -429,7 +429,7 @@ namespace sci_cuda {
                         for (int c = 0; c < 32; c += 4) vector(published + q * kSmallPitch + c) = make_float4(w[c], w[c + 1], w[c + 2], w[c + 3]);
                     }
                     __syncthreads();
-                    product(K);
+                    substitute(K);
                     __syncthreads();
                     auto subtract_row = [&](int k, float l) {
                         const unsigned long long f = small_pair(-l, -l);
@@ -483,7 +483,7 @@ namespace sci_cuda {
                 if (row && place >= j0 && place < j0 + bw) {
 #pragma unroll
                     for (int c = 0; c < 32; c += 4)
-                        vector(u_block + (place - j0) * kSmallPitch + c) = make_float4(kept[c], kept[c + 1], kept[c + 2], kept[c + 3]);
+                        vector(triangle_row(J, place - j0) + c) = make_float4(kept[c], kept[c + 1], kept[c + 2], kept[c + 3]);
                 }
             } else {
                 if (J > 0) {
@@ -515,7 +515,7 @@ namespace sci_cuda {
                             }
                         }
                         __syncthreads();
-                        product(K);
+                        substitute(K);
                         __syncthreads();
                         if (__any_sync(kAll, below)) {
 #pragma unroll 2
@@ -592,117 +592,6 @@ namespace sci_cuda {
                 }
                 __syncthreads();
                 if (row) place = places[tid];
-                // the block's L and U (bordered by the identity), for the warps that invert them
-                for (int piece = tid; piece < 8 * bw; piece += blockDim.x) {
-                    const int i = piece >> 3, c = (piece & 7) * 4;
-                    vector(u_block + i * kSmallPitch + c) = j0 + c < columns ? vector(A + rows[j0 + i] * P + j0 + c)
-                                                                             : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
-            }
-            for (int i = bw + warp; i < 32; i += warps) u_block[i * kSmallPitch + lane] = lane == i ? 1.0f : 0.0f;
-            __syncthreads();
-            // Both inverses in place, a warp each: the two 16 x 16 diagonal blocks side by side (a lane per column), then the
-            // block between them from the products -X22 (L21 X11) and -Y11 (U12 Y22).
-            auto corner = [&](bool lower) {
-                const int r0 = (lane >> 3) * 4, c0 = (lane & 7) * 2;  // four rows and two columns of the 16 x 16 products
-                float *scratch = published + (lower ? 0 : 16) * kSmallPitch;
-#pragma unroll 1
-                for (int step = 0; step < 2; ++step) {
-                    // first: the off-diagonal block times the inverse of its column's diagonal block; then the inverse of its
-                    // row's diagonal block times that
-                    const bool off = step == 0;
-                    const float *left = off ? (lower ? u_block + 16 * kSmallPitch : u_block + 16)
-                                            : (lower ? u_block + 16 * kSmallPitch + 16 : u_block);
-                    const float *right = off ? (lower ? u_block : u_block + 16 * kSmallPitch + 16) : scratch;
-                    float acc[4][2] = {};
-#pragma unroll
-                    for (int k0 = 0; k0 < 16; k0 += 4) {
-                        float b[4][2];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int k = k0 + e;
-                            const float2 v = *reinterpret_cast<const float2 *>(right + k * kSmallPitch + c0);
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const float entry = h == 0 ? v.x : v.y;
-                                const int c = c0 + h;
-                                b[e][h] = !off ? entry : (lower ? (k > c ? entry : (k == c ? 1.0f : 0.0f)) : (k <= c ? entry : 0.0f));
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const float4 v = *reinterpret_cast<const float4 *>(left + (r0 + i) * kSmallPitch + k0);
-                            const float line[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int k = k0 + e, at = r0 + i;
-                                const float l = off ? line[e] : (lower ? (k < at ? line[e] : (k == at ? 1.0f : 0.0f)) : (k >= at ? line[e] : 0.0f));
-                                acc[i][0] = fmaf(l, b[e][0], acc[i][0]);
-                                acc[i][1] = fmaf(l, b[e][1], acc[i][1]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-                    float *out = off ? scratch : (lower ? u_block + 16 * kSmallPitch : u_block + 16);
-                    const float sign = off ? 1.0f : -1.0f;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        *reinterpret_cast<float2 *>(out + (r0 + i) * kSmallPitch + c0) = make_float2(sign * acc[i][0], sign * acc[i][1]);
-                    __syncwarp();
-                }
-            };
-            const int side = lane & 16, at = lane & 15;  // this lane's diagonal block, and its column of it
-            float *diagonal = u_block + side * kSmallPitch + side;
-            if (warp == 0) {
-                float v[16];
-                static_for<16>([&](auto i_c) {
-                    constexpr int i = decltype(i_c)::value;
-                    float s[4] = {at == i ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                    for (int k = 0; k < i; k += 4) {
-                        const float4 l = vector(diagonal + i * kSmallPitch + k);
-                        s[0] = fmaf(-l.x, v[k], s[0]);
-                        if (k + 1 < i) s[1] = fmaf(-l.y, v[k + 1], s[1]);
-                        if (k + 2 < i) s[2] = fmaf(-l.z, v[k + 2], s[2]);
-                        if (k + 3 < i) s[3] = fmaf(-l.w, v[k + 3], s[3]);
-                    }
-                    v[i] = (s[0] + s[1]) + (s[2] + s[3]);
-                });
-                __syncwarp();
-#pragma unroll
-                for (int i = 1; i < 16; ++i)
-                    if (at < i) diagonal[i * kSmallPitch + at] = v[i];
-                __syncwarp();
-                corner(true);
-            }
-            if (warp == (warps > 1 ? 1 : 0)) {
-                float v[16];
-                const float reciprocal = div(1.0f, u_block[lane * kSmallPitch + lane]);
-                static_for<16>([&](auto i_c) {
-                    constexpr int i = 15 - decltype(i_c)::value;
-                    float s[4] = {at == i ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-                    for (int k = i / 4 * 4; k < 16; k += 4) {
-                        const float4 u = vector(diagonal + i * kSmallPitch + k);
-                        if (k > i) s[0] = fmaf(-u.x, v[k], s[0]);
-                        if (k + 1 > i) s[1] = fmaf(-u.y, v[k + 1], s[1]);
-                        if (k + 2 > i) s[2] = fmaf(-u.z, v[k + 2], s[2]);
-                        if (k + 3 > i) s[3] = fmaf(-u.w, v[k + 3], s[3]);
-                    }
-                    v[i] = ((s[0] + s[1]) + (s[2] + s[3])) * __shfl_sync(kAll, reciprocal, side + i);
-                });
-                __syncwarp();
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (at >= i) diagonal[i * kSmallPitch + at] = v[i];
-                __syncwarp();
-                corner(false);
-            }
-            __syncthreads();
-            // home: over the block's own rows
-            for (int piece = tid; piece < 8 * bw; piece += blockDim.x) {
-                const int i = piece >> 3, c = (piece & 7) * 4;
-                if ((RB > 0 && J >= SB) || j0 + c < columns) vector(inverse_row(J, i) + c) = vector(u_block + i * kSmallPitch + c);
             }
         }
         __syncthreads();
@@ -746,30 +635,55 @@ namespace sci_cuda {
                 }
             }
         };
-        // the product of lane's row of block K's inverse (its entries before `lane` for L, from it on for U) with the block's
-        // right-hand sides; zeros for lanes beyond the block
-        auto solve_block = [&](int K, int bw, bool lower, float (&y)[NR]) {
-            const float *inverse = inverse_row(K, lane < bw ? lane : 0);
-            float s[2][NR];
+        // Block K's right-hand sides by substitution, a row per lane of one warp: four columns at a time, whose own
+        // 4 x 4 triangle every lane solves for itself, so that the chain crosses the lanes eight times, not 32. U's rows
+        // are divided by their diagonals first. Zeros for lanes beyond the block.
+        auto solve_block = [&](int K, int bw, auto lower_c, float (&y)[NR]) {
+            constexpr bool lower = decltype(lower_c)::value != 0;
+            float *own_line = triangle_row(K, lane < bw ? lane : 0);
+            Divisor own{};
+            if constexpr (!lower) own = divisor_of(own_line[lane < bw ? lane : 0]);
 #pragma unroll
-            for (int q = 0; q < NR; ++q) s[0][q] = lower ? to_solve[lane * NR + q] : 0.0f, s[1][q] = 0.0f;
-            // all loads first; what lies beyond the block's columns is another row's (or nothing's) and is dropped
-            float4 line[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) line[k] = *reinterpret_cast<const float4 *>(inverse + 4 * k);
-#pragma unroll
-            for (int k0 = 0; k0 < 32; k0 += 4) {
-                const float l[4] = {line[k0 / 4].x, line[k0 / 4].y, line[k0 / 4].z, line[k0 / 4].w};
+            for (int q = 0; q < NR; ++q) {
+                y[q] = lane < bw ? to_solve[lane * NR + q] : 0.0f;
+                if constexpr (!lower) y[q] = lane < bw ? quotient_of(y[q], own) : 0.0f;
+            }
+            const int groups = (bw + 3) / 4;
+            float4 next = vector(own_line + (lower ? 0 : 4 * groups - 4));
+#pragma unroll 2
+            for (int step = 0; step < groups; ++step) {
+                const int g = lower ? step : groups - 1 - step;
+                float pieces[4] = {next.x, next.y, next.z, next.w};
+                if (step + 1 < groups) next = vector(own_line + 4 * (lower ? g + 1 : g - 1));
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int k = k0 + e;
-                    const float f = (lower ? k < lane : (k >= lane && k < bw)) ? l[e] : 0.0f;
+                    // what lies beyond the triangle, or the block's columns (another row's, or nothing's), counts as zero
+                    const int k = 4 * g + e;
+                    const bool inside = lower ? k < lane && lane < bw : k > lane && k < bw;
+                    if constexpr (lower) pieces[e] = inside ? -pieces[e] : 0.0f;
+                    else pieces[e] = inside ? -quotient_of(pieces[e], own) : 0.0f;
+                }
+                float t[4][NR];
 #pragma unroll
-                    for (int q = 0; q < NR; ++q) s[e & 1][q] = fmaf(f, to_solve[k * NR + q], s[e & 1][q]);
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) t[e][q] = __shfl_sync(kAll, y[q], 4 * g + e);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int e = lower ? u : 3 - u;
+#pragma unroll
+                    for (int f = 0; f < 4; ++f) {
+                        if (lower ? f <= e : f >= e) continue;
+                        const float entry = __shfl_sync(kAll, pieces[e], 4 * g + f);
+#pragma unroll
+                        for (int q = 0; q < NR; ++q) t[f][q] = fmaf(entry, t[e][q], t[f][q]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < NR; ++q) y[q] = fmaf(pieces[e], t[e][q], y[q]);
                 }
             }
 #pragma unroll
-            for (int q = 0; q < NR; ++q) y[q] = lane < bw ? s[0][q] + s[1][q] : 0.0f;
+            for (int q = 0; q < NR; ++q) y[q] = lane < bw ? y[q] : 0.0f;
         };
         while (true) {
 #pragma unroll 1
@@ -785,7 +699,7 @@ namespace sci_cuda {
                 if (below) entries(K, l);
                 if (warp == 0) {
                     float y[NR];
-                    solve_block(K, bw, true, y);
+                    solve_block(K, bw, Int<1>{}, y);
 #pragma unroll
                     for (int q = 0; q < NR; ++q) solved[lane * NR + q] = y[q];
                 }
@@ -809,7 +723,7 @@ namespace sci_cuda {
                 if (at < 0) entries(K, l);  // the rows placed above the block
                 if (warp == 0) {
                     float y[NR];
-                    solve_block(K, bw, false, y);
+                    solve_block(K, bw, Int<0>{}, y);
 #pragma unroll
                     for (int q = 0; q < NR; ++q) {
                         solved[lane * NR + q] = y[q];
