@@ -733,33 +733,37 @@ namespace sci_cuda {
                 __syncthreads();
                 if (at < 0) subtract(l);
             }
-            // r = b - A x in FP64, with |r_q|_inf and |x_q|_inf
+            // r = b - A x in FP64, with |r_q|_inf and |x_q|_inf. The diagonal's term is subtracted from b first, by the row's
+            // thread: in diagonally dominant systems they nearly cancel, and what is added to them rounds at the
+            // remainder's size (orders 16 to 256, A = G + nI: a mean backward error of 4.8e-17 to 9.6e-17 with
+            // the term in the row's sum, 2.1e-17 to 2.4e-17 here).
             double left[NR], r_max[NR], x_max[NR];  // this row's residuals
+            const double diagonal = row ? a[1ll * tid * n + tid] : 0.0;
 #pragma unroll
-            for (int q = 0; q < NR; ++q) left[q] = 0.0;
+            for (int q = 0; q < NR; ++q) left[q] = row ? fma(-diagonal, x[tid * NR + q], rhs[q]) : 0.0;
             if (sys.transposed) {
+                // A thread per row, in parts of 16 terms whose sums are added to the total: a rounding error for every 16
+                // terms or less, as in the blocked residual (one chain over all terms doubled the error at order 256).
                 if (row) {
-                    double s[NR][2];
+                    auto part = [&](int k0, auto whole_c) {
+                        constexpr bool whole = decltype(whole_c)::value != 0;
+                        double v[16], s[NR][2];
 #pragma unroll
-                    for (int q = 0; q < NR; ++q) s[q][0] = s[q][1] = 0.0;
-#pragma unroll 8
-                    for (int k = 0; k + 1 < n; k += 2) {
-                        const double v0 = a[1ll * k * n + tid], v1 = a[1ll * (k + 1) * n + tid];
+                        for (int k = 0; k < 16; ++k) v[k] = (whole || k0 + k < n) && k0 + k != tid ? a[1ll * (k0 + k) * n + tid] : 0.0;
 #pragma unroll
-                        for (int q = 0; q < NR; ++q) {
-                            s[q][0] = fma(v0, x[k * NR + q], s[q][0]);
-                            s[q][1] = fma(v1, x[(k + 1) * NR + q], s[q][1]);
-                        }
-                    }
-                    if (n & 1) {
-                        const double v = a[1ll * (n - 1) * n + tid];
+                        for (int q = 0; q < NR; ++q) s[q][0] = s[q][1] = 0.0;
 #pragma unroll
-                        for (int q = 0; q < NR; ++q) s[q][0] = fma(v, x[(n - 1) * NR + q], s[q][0]);
-                    }
+                        for (int k = 0; k < 16; ++k)
 #pragma unroll
-                    for (int q = 0; q < NR; ++q) {
-                        left[q] = rhs[q] - (s[q][0] + s[q][1]);
-                    }
+                            for (int q = 0; q < NR; ++q)
+                                s[q][k & 1] = fma(v[k], whole || k0 + k < n ? x[(k0 + k) * NR + q] : 0.0, s[q][k & 1]);
+#pragma unroll
+                        for (int q = 0; q < NR; ++q) left[q] -= s[q][0] + s[q][1];
+                    };
+                    int k0 = 0;
+#pragma unroll 2
+                    for (; k0 + 16 <= n; k0 += 16) part(k0, Int<1>{});
+                    if (k0 < n) part(k0, Int<0>{});
                 }
             } else {
                 // a warp per row, several rows' loads in flight (as the load); R rows' sums of every right-hand side
@@ -772,7 +776,7 @@ namespace sci_cuda {
 #pragma unroll
                             for (int g = 0; g < G; ++g) {
                                 const int at = row0 + u * warps, col = lane + 32 * g;
-                                v[u][g] = at < n && col < n ? a[1ll * at * n + col] : 0.0;
+                                v[u][g] = at < n && col < n && col != at ? a[1ll * at * n + col] : 0.0;
                             }
                     };
                     fetch(warp);
@@ -804,7 +808,7 @@ namespace sci_cuda {
                 __syncthreads();
                 if (row) {
 #pragma unroll
-                    for (int q = 0; q < NR; ++q) left[q] = rhs[q] - sums[tid * NR + q];
+                    for (int q = 0; q < NR; ++q) left[q] -= sums[tid * NR + q];
                 }
             }
 #pragma unroll
