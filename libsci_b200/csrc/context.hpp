@@ -217,8 +217,8 @@ namespace sci_cuda {
     // Row-major GEMMs on submatrices (product.cu): C (pitch ldc) = A (pitch lda) * B (pitch ldb),
     // or C -= A * B with `subtract`. tensor_gemm splits each operand into `terms` (1-3) bf16 parts
     // and multiplies on the tensor cores; simt_gemm is the plain FP32 / FP64 form. Both queue on
-    // ctx.stream. `whole_gpu`: the product has the GPU to itself, so it
-    // runs on the persistent CTA-pair kernel (a static split of the tiles over every SM); the LU's
+    // ctx.stream. `whole_gpu`: the product has the GPU to itself, so it runs on the persistent CTA-pair
+    // kernel (a static split of the tiles over every SM; a bf16 product of few rows on single CTAs); the LU's
     // updates, which share the GPU with the panels, keep the one-tile-per-CTA kernel. `chained`: the
     // first launch follows the kernel before it on the stream directly, so the conversions and the
     // product are launched with programmatic stream serialization (each waits for the one before).

@@ -32,6 +32,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <utility>
 
 namespace sci_cuda {
 
@@ -226,6 +227,7 @@ namespace sci_cuda {
             unsigned long long m, n, kp, ldc;
             int subtract;  // C -= A B instead of C = A B
             int *status;
+            int flipped;  // the pair kernel computes C^T: m and n are C's columns and rows
             // the pair kernel's split depth: pieces of `span` k-blocks, their sums in `partial`, a ticket per tile and warp
             unsigned pieces, span;
             float *partial;
@@ -661,7 +663,7 @@ namespace sci_cuda {
                         // subtracting update) combine with what C holds
                         const int how = args.subtract ? -1 : (k0 == first ? 0 : 1);
 #pragma unroll 1
-                        for (int chunk = 0; chunk < BN / 32; ++chunk) {
+                        for (int chunk = 0; chunk < BN / 32 && n0 + chunk * 32 < args.n; ++chunk) {
                             unsigned v[32];
                             const unsigned address = tmem + ((warp * 32u) << 16) + b * Sh::buffer + chunk * 32u;
                             tmem_load32(address, v);
@@ -689,6 +691,21 @@ namespace sci_cuda {
                                         }
                                         *reinterpret_cast<float4 *>(dst + j) = out;
                                     }
+                                }
+                            } else if (Sh::split && args.flipped) {
+                                // a column of the tile per store: the lanes lie along a row of C
+                                if (row < args.m) {
+                                    float *const dst = args.c + col * args.ldc + row;
+                                    if (how != 0) {
+                                        float old[32];
+#pragma unroll
+                                        for (int j = 0; j < 32; ++j) old[j] = col + j < args.n ? dst[j * args.ldc] : 0.0f;
+#pragma unroll
+                                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(old[j] + __uint_as_float(v[j]));
+                                    }
+#pragma unroll
+                                    for (int j = 0; j < 32; ++j)
+                                        if (col + j < args.n) dst[j * args.ldc] = __uint_as_float(v[j]);
                                 }
                             } else if (row < args.m && col < args.n) {
                                 float *dst = args.c + row * args.ldc + col;
@@ -943,32 +960,55 @@ namespace sci_cuda {
         const unsigned long long kp = (k + kBK - 1) / kBK * kBK;
         if (kp > (1ull << 31) || m > (1ull << 31) || n > (1ull << 31))
             return ctx.fail(SCI_CUDA_ERROR_UNSUPPORTED, "product dimensions beyond 2^31");
-        const unsigned long long a_bytes = (m * kp * 2 + 1023) / 1024 * 1024, b_bytes = (n * kp * 2 + 1023) / 1024 * 1024;
         // The pair kernel's tiles, and the pieces their depth is cut into: as many as give every pair an item, as long as
         // that is quicker. A k-block takes about 0.13 us per product of terms and the last warp's pass over
         // one piece's tile about 0.75 us, so span / pieces x products x 0.13 + pieces x 0.75 is least
-        // where pieces^2 = span x products / 6. (bf16 500 x 500 x 4000, four tiles: 41 us in one piece, 53 in 15.)
-        const bool paired = whole_gpu && pair_kernel_enabled();
+        // where pieces^2 = span x products / 6. (bf16 500 x 500 x 4000, four tiles: 41 us in one piece, 53 in 15.) One
+        // term in two pieces breaks even at 48 k-blocks (128 x 64: 23 us in one, 27 in two at 32 k-blocks, 29 and
+        // 25 at 63).
+        bool paired = whole_gpu && pair_kernel_enabled();
         const unsigned pair_bn = terms == 1 ? PairShape<1>::BN : PairShape<3>::BN;
-        unsigned tiles_m = static_cast<unsigned>((m + 255) / 256), tiles_n = static_cast<unsigned>((n + pair_bn - 1) / pair_bn);
         const void *pair_kernel = terms == 1 ? reinterpret_cast<const void *>(&tensor_product_pair<1>)
                                 : terms == 2 ? reinterpret_cast<const void *>(&tensor_product_pair<2>)
                                              : reinterpret_cast<const void *>(&tensor_product_pair<3>);
         const size_t pair_smem = terms == 1 ? PairShape<1>::stages * PairShape<1>::stage + 1024
                                : terms == 2 ? PairShape<2>::stages * PairShape<2>::stage + 1024
                                             : PairShape<3>::stages * PairShape<3>::stage + 1024;
-        const unsigned long long tiles = 1ull * tiles_m * tiles_n;
+        const unsigned long long products = terms == 1 ? 1 : (terms == 2 ? 3 : 6);
         unsigned long long slots = 0, pieces = 1, span = kp / kBK;
+        bool flipped = false;
         if (paired) {
             if (int code = ctx.check(cudaFuncSetAttribute(pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                           static_cast<int>(pair_smem)),
                                      "raising the pair kernel's shared memory"))
                 return code;
             slots = pair_slots(pair_kernel, pair_smem, ctx.sms);
-            const unsigned long long products = terms == 1 ? 1 : (terms == 2 ? 3 : 6);
-            while (!subtract && (pieces + 1) * tiles <= slots && 6 * (pieces + 1) * (pieces + 1) <= span * products) ++pieces;
+            // C of at most 128 rows and more tiles than pairs: half of each 256-row tile would be padding, so the kernel
+            // computes C^T = B^T A^T instead, in tiles of 256 of C's columns, and stores it along C's rows. 128 x 30000 x
+            // 4000: 546 -> 434 us with three terms, 394 -> 333 with two. Not above 64 rows of a short depth: that is
+            // bound by the stores, which this makes no quicker (two terms 128 x 60000 x 256: 83 us, 85 this way).
+            flipped = terms > 1 && !subtract && m <= 128 && (n + pair_bn - 1) / pair_bn > slots && (m <= 64 || span * products >= 48);
+            if (flipped) {
+                std::swap(a, b);
+                std::swap(lda, ldb);
+                std::swap(m, n);
+                const bool stored = a_t;
+                a_t = !b_t;
+                b_t = !stored;
+            }
+        }
+        const unsigned long long a_bytes = (m * kp * 2 + 1023) / 1024 * 1024, b_bytes = (n * kp * 2 + 1023) / 1024 * 1024;
+        unsigned tiles_m = static_cast<unsigned>((m + 255) / 256), tiles_n = static_cast<unsigned>((n + pair_bn - 1) / pair_bn);
+        const unsigned long long tiles = 1ull * tiles_m * tiles_n;
+        if (paired) {
+            const auto least = [&](unsigned long long cut) { return terms == 1 && cut == 2 ? 48 : 6 * cut * cut; };
+            while (!subtract && (pieces + 1) * tiles <= slots && least(pieces + 1) <= span * products) ++pieces;
             span = (span + pieces - 1) / pieces;
             pieces = (kp / kBK + span - 1) / span;
+            // One term, at most 128 rows, no pieces: tiles of 128 rows on single CTAs, which add in the same order (64 x 2048 x
+            // 2000: 29 -> 23 us; 128 x 60000 x 256: 69 -> 52; 128 x 30000 x 4000: 226 -> 217). With more terms that
+            // kernel's single accumulator is less accurate.
+            if (terms == 1 && m <= 128 && pieces == 1) paired = false;
         }
         const unsigned long long tile_bytes = 256ull * pair_bn * 4;
         const unsigned long long partial_bytes = pieces > 1 ? tiles * pieces * tile_bytes + tiles * 8 * 4 : 0;
@@ -1008,12 +1048,11 @@ namespace sci_cuda {
         SplitJob job_a = job(a, lda, at, m, a_t), job_b = job(b, ldb, bt, n, !b_t);
         int term_count = terms;
         void *split_params[] = {&job_a, &job_b, &term_count, &tickets, &ticket_count};
-        if (int code = ctx.check(launch(reinterpret_cast<const void *>(&split_operands), dim3(job_a.blocks + job_b.blocks), dim3(256),
-                                        split_params, 0, chained),
+        if (int code = ctx.check(launch(reinterpret_cast<const void *>(&split_operands), dim3(job_a.blocks + job_b.blocks), dim3(256), split_params, 0, chained),
                                  "launching the bf16 conversion"))
             return code;
 
-        ProductArgs args{c, m, n, kp, ldc, subtract ? 1 : 0, ctx.status, static_cast<unsigned>(pieces), static_cast<unsigned>(span),
+        ProductArgs args{c, m, n, kp, ldc, subtract ? 1 : 0, ctx.status, flipped ? 1 : 0, static_cast<unsigned>(pieces), static_cast<unsigned>(span),
                          partial, tickets};
         if (paired) {
             // 256 x 256 (one term) or 256 x 128 tiles on CTA pairs, persistent
@@ -1047,7 +1086,7 @@ namespace sci_cuda {
             return code;
         void *params[] = {&maps, &args};
         const dim3 pgrid(static_cast<unsigned>((n + bn - 1) / bn), static_cast<unsigned>((m + kBM - 1) / kBM));
-        return ctx.check(launch(kernel, pgrid, dim3(192), params, smem, chained), "launching the tensor product");
+        return ctx.check(launch(kernel, pgrid, dim3(192), params, smem, chained || whole_gpu), "launching the tensor product");
     }
 
     // C (pitch ldc) = or -= A (pitch lda) * B (pitch ldb) with the plain SIMT kernel; a_t / b_t as for
