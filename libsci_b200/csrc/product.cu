@@ -149,7 +149,11 @@ namespace sci_cuda {
         // Both operands in one launch (a launch of its own for each took 4 to 7 us at orders around 1000, most of it
         // starting and ending): the first blocks convert A, the others B. It also clears the tickets of
         // a product whose depth is split.
-        __global__ void __launch_bounds__(256) split_operands(const __grid_constant__ SplitJob a, const __grid_constant__ SplitJob b,
+        // LARGE operands (more than 32 MB) go at eight blocks per SM, as the memory's latency needs (39 registers leave six:
+        // 1 x 30000 x 4000 in one term, nearly all of it conversion, 221 -> 206 us; 128 x 8192 x 2000 44 -> 42); for
+        // few blocks the registers are worth more (512^3 16.0 us with 39 registers, 16.9 with 32).
+        template <bool LARGE>
+        __global__ void __launch_bounds__(256, LARGE ? 8 : 6) split_operands(const __grid_constant__ SplitJob a, const __grid_constant__ SplitJob b,
                                                               int terms, unsigned *tickets, unsigned ticket_count) {
             __shared__ float tile[64][65];
             follow_previous();
@@ -1048,7 +1052,9 @@ namespace sci_cuda {
         SplitJob job_a = job(a, lda, at, m, a_t), job_b = job(b, ldb, bt, n, !b_t);
         int term_count = terms;
         void *split_params[] = {&job_a, &job_b, &term_count, &tickets, &ticket_count};
-        if (int code = ctx.check(launch(reinterpret_cast<const void *>(&split_operands), dim3(job_a.blocks + job_b.blocks), dim3(256), split_params, 0, chained),
+        const bool large = (m + n) * k * 4 > (32ull << 20);
+        const void *split = large ? reinterpret_cast<const void *>(&split_operands<true>) : reinterpret_cast<const void *>(&split_operands<false>);
+        if (int code = ctx.check(launch(split, dim3(job_a.blocks + job_b.blocks), dim3(256), split_params, 0, chained),
                                  "launching the bf16 conversion"))
             return code;
 
