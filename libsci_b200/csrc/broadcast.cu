@@ -16,11 +16,11 @@
 //
 // Kernels: the host merges adjacent axes that every operand reads alike (both broadcast or both
 // full), so most calls reduce to one or two axes (a same-shape or scalar operation to one). When
-// the last merged axis is 64 elements or more, blocks walk (row, piece of the last axis) pairs: the
-// row's offsets are computed once per piece and the piece is read and written contiguously
-// (stride 0 or 1 per operand) in 16-byte vectors, two per thread. Shorter last axes map each
-// thread's flat index to every operand's offset. HBM bound: bytes = the output written + each
-// operand read once (a broadcast operand mostly from L2).
+// the last merged axis is long, blocks walk (row, piece of the last axis) pairs: the row's offsets
+// are computed once per piece and the piece is read and written contiguously (stride 0 or 1 per
+// operand), in 16-byte vectors, two per thread, or element by element. Short last axes map each
+// thread's flat index to every operand's offset (launch_apply says where the lines lie). HBM bound:
+// bytes = the output written + each operand read once (a broadcast operand mostly from L2).
 #include "context.hpp"
 
 #include <cuda_runtime.h>
@@ -33,6 +33,7 @@ namespace sci_cuda {
     namespace {
 
         constexpr int kMaxAxes = 8;
+        constexpr unsigned kPiece = 1024;
         constexpr int kVectorsPerThread = 2;  // 16-byte vectors per thread per piece (vector form)
 
         template <typename T> struct ApplyLaunch {
@@ -94,6 +95,31 @@ namespace sci_cuda {
             }
         }
 
+        // Rows: (row, piece of the last axis) per block step; the last axis is read with stride 0
+        // or 1 per operand.
+        template <typename T> __global__ void __launch_bounds__(256) apply_rows(const __grid_constant__ ApplyLaunch<T> L) {
+            const int last = L.rank - 1;
+            const unsigned long long columns = L.extent[last];
+            const unsigned long long chunks = (columns + kPiece - 1) / kPiece;
+            const unsigned long long rows = L.count / columns, pieces = rows * chunks;
+            for (unsigned long long piece = blockIdx.x; piece < pieces; piece += gridDim.x) {
+                const unsigned long long row = piece / chunks, c0 = (piece - row * chunks) * kPiece;
+                unsigned long long rest = row, base[3] = {0, 0, 0};
+                for (int axis = last - 1; axis >= 0; --axis) {
+                    const unsigned long long coordinate = rest % L.extent[axis];
+                    rest /= L.extent[axis];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) base[k] += coordinate * L.stride[k][axis];
+                }
+                T *out = L.output + row * columns;
+                for (unsigned long long c = c0 + threadIdx.x; c < c0 + kPiece && c < columns; c += blockDim.x) {
+                    out[c] = apply_shaped<T>(L.code, operand(L, 0, base[0] + c * L.stride[0][last]),
+                                             operand(L, 1, base[1] + c * L.stride[1][last]),
+                                             operand(L, 2, base[2] + c * L.stride[2][last]));
+                }
+            }
+        }
+
         // Rows in 16-byte vectors, two per thread per piece, whatever the row length and the arrays'
         // alignment: a row's vectors start at the first element that lies on a 16-byte boundary of
         // the output, and the few elements before and after them are done one by one. An
@@ -112,7 +138,7 @@ namespace sci_cuda {
             constexpr unsigned V = 16 / sizeof(T), U = kVectorsPerThread;
             const int last = L.rank - 1;
             const unsigned long long columns = L.extent[last], span = 256ull * V * U;
-            const unsigned long long chunks = (columns + (EVEN ? 0 : V - 1) + span - 1) / span;  // up to V - 1 elements come before the vectors
+            const unsigned long long chunks = (columns + span - 1) / span;  // at most columns / V vectors after the row's first boundary
             const unsigned long long rows = L.count / columns;
             const unsigned long long row_step = gridDim.x / chunks, chunk_step = gridDim.x - row_step * chunks;
             unsigned long long row = blockIdx.x / chunks, chunk = blockIdx.x - row * chunks;
@@ -178,17 +204,20 @@ namespace sci_cuda {
         template <typename T, int CODE, bool EVEN> void launch_vectors(Context &ctx, const ApplyLaunch<T> &L) {
             constexpr int V = 16 / sizeof(T);
             const unsigned long long columns = L.extent[L.rank - 1], span = 256ull * V * kVectorsPerThread;
-            const unsigned long long pieces = (L.count / columns) * ((columns + (EVEN ? 0 : V - 1) + span - 1) / span);
+            const unsigned long long pieces = (L.count / columns) * ((columns + span - 1) / span);
             // one wave: as many blocks as stay resident
             const unsigned long long most =
                     1ull * ctx.sms * ctx.blocks_per_sm(reinterpret_cast<const void *>(&apply_vectors<T, CODE, EVEN>), 256, 0);
             apply_vectors<T, CODE, EVEN><<<static_cast<unsigned>(pieces < most ? pieces : most), 256, 0, ctx.stream>>>(L);
         }
-        template <typename T, int CODE> void launch_vectors(Context &ctx, const ApplyLaunch<T> &L) {
+        // Rows of whole vectors in aligned arrays: every row starts on a vector.
+        template <typename T> bool even(const ApplyLaunch<T> &L) {
             auto aligned = [](const void *p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
-            if (L.extent[L.rank - 1] % (16 / sizeof(T)) == 0 && aligned(L.output) && aligned(L.input[0]) && aligned(L.input[1]) &&
-                aligned(L.input[2]))
-                launch_vectors<T, CODE, true>(ctx, L);
+            return L.extent[L.rank - 1] % (16 / sizeof(T)) == 0 && aligned(L.output) && aligned(L.input[0]) && aligned(L.input[1]) &&
+                   aligned(L.input[2]);
+        }
+        template <typename T, int CODE> void launch_vectors(Context &ctx, const ApplyLaunch<T> &L) {
+            if (even(L)) launch_vectors<T, CODE, true>(ctx, L);
             else launch_vectors<T, CODE, false>(ctx, L);
         }
 
@@ -234,11 +263,22 @@ namespace sci_cuda {
             }
             L.output = static_cast<T *>(output);
             L.count = count;
-            // Rows shorter than 64 elements leave most of a block without a vector: a flat index per element there.
-            if (extent[rank - 1] >= 64) {
+            // A block of the row forms steps from row to row, so short rows leave most of it idle. Rows of whole vectors go by
+            // vectors from 64 elements on. Ragged ones by a flat index below 288 (where((r, 1), x, y) of 500000 x 127
+            // floats: 480 us flat, 970 by rows, 1903 by vectors), from there by vectors (100000 x 385, (r, 1) + (1, c): 185,
+            // 256 flat, 213 by rows) -- but three operands by rows below 576 (the same size: 307 by rows, 294 flat, 359
+            // by vectors; 40000 x 1023: 150 by vectors, 221 by rows), and powers, which are bound by their arithmetic,
+            // by rows below 16384 (20000 x 2049 floats: 497 by rows, 912 by vectors; 30 x 2000003: 695 and 632).
+            const unsigned long long columns = extent[rank - 1];
+            const unsigned long long most = 8ull * ctx.sms;
+            const unsigned long long vectors_from = code == SCI_EXTRA_POWER ? 16384 : (operands == 3 ? 576 : 288);
+            if (columns >= 64 && (even(L) || columns >= vectors_from)) {
                 launch_vector_code<T>(ctx, L);
+            } else if (columns >= 288) {
+                const unsigned long long pieces = (count / columns) * ((columns + kPiece - 1) / kPiece);
+                apply_rows<T><<<static_cast<unsigned>(pieces < most ? pieces : most), 256, 0, ctx.stream>>>(L);
             } else {
-                const unsigned long long wanted = (count + 255) / 256, most = 8ull * ctx.sms;
+                const unsigned long long wanted = (count + 255) / 256;
                 apply_flat<T><<<static_cast<unsigned>(wanted < most ? wanted : most), 256, 0, ctx.stream>>>(L);
             }
             return ctx.check(cudaGetLastError(), "launching a broadcast operation");
