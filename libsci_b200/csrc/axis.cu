@@ -14,7 +14,7 @@
 //     per k -- or, when inner is a whole number of 16-byte vectors, a thread per (o, piece, vector
 //     of j) reading 512 bytes per warp per k (rows shorter than 64 take this form, a thread
 //     per row).
-// Each lane keeps 8 to 16 loads in flight ahead of its ordered fold, and the kind of fold is a template
+// Each lane keeps 4 to 16 loads in flight ahead of its ordered fold, and the kind of fold is a template
 // argument. Sum over axis 0 and mean over axis 1 of 16384 x 16384 floats (one call, events around
 // it): 233 -> 189 us (5.7 TB/s) and 199 -> 184; of 5001 x 7003: 54 -> 47 and 45 -> 38. A block per 128
 // columns, its warps' folds combined in shared memory, took 370 us for the first (512 bytes of a row
@@ -22,12 +22,14 @@
 // Short outputs over long axes split the axis
 // into pieces so the grid fills the GPU; pieces write
 // double partials that one more pass folds in piece order. The order of every fold is fixed by the
-// shape alone, so results are deterministic. HBM bound: the input is read once.
+// shape, the input's 16-byte alignment (vectors or single columns) and the GPU (the pieces fill its
+// waves), so results are deterministic. HBM bound: the input is read once.
 #include "context.hpp"
 #include "workspace.hpp"
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <limits>
 
 using namespace sci_cuda;
@@ -66,9 +68,8 @@ namespace sci_cuda {
             unsigned folded;  // the fold applied to values (mean folds as a sum)
         };
 
-        template <typename T, unsigned FOLD>
+        template <typename T, unsigned FOLD, int U>
         __global__ void __launch_bounds__(256) axis_rows(const T *in, AxisShape s, double *partial, T *out) {
-            constexpr int U = 16;  // loads in flight per lane
             const unsigned lane = threadIdx.x & 31;
             const unsigned long long warps = 1ull * gridDim.x * (blockDim.x >> 5);
             const unsigned long long units = s.outer * s.pieces;
@@ -149,15 +150,23 @@ namespace sci_cuda {
         }
 
         // Folds the pieces of every output in piece order: partial[(o * pieces + p) * inner + j].
-        template <typename T>
+        template <typename T, unsigned FOLD>
         __global__ void __launch_bounds__(256) axis_pieces(const double *partial, AxisShape s, T *out) {
             const unsigned long long outputs = s.outer * s.inner, step = 1ull * gridDim.x * blockDim.x;
             for (unsigned long long i = 1ull * blockIdx.x * blockDim.x + threadIdx.x; i < outputs; i += step) {
                 const unsigned long long o = i / s.inner, j = i - o * s.inner;
-                double acc = fold_start(s.folded);
-                // eight loads in flight ahead of the (ordered) fold
-#pragma unroll 8
-                for (unsigned long long p = 0; p < s.pieces; ++p) acc = fold_pair(s.folded, acc, partial[(o * s.pieces + p) * s.inner + j]);
+                double acc = fold_start(FOLD);
+                const double *from = partial + o * s.pieces * s.inner + j;
+                constexpr int U = 16;  // loads in flight ahead of the (ordered) fold
+                unsigned long long p = 0;
+                for (; p + U <= s.pieces; p += U) {
+                    double v[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v[u] = from[(p + u) * s.inner];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) acc = fold_pair(FOLD, acc, v[u]);
+                }
+                for (; p < s.pieces; ++p) acc = fold_pair(FOLD, acc, from[p * s.inner]);
                 out[i] = finish<T>(s.fold, acc, s.extent);
             }
         }
@@ -168,22 +177,37 @@ namespace sci_cuda {
             constexpr int V = 16 / sizeof(T);
             const bool rows = s.inner == 1 && s.extent >= 64;  // shorter rows go a thread per row
             const bool vectors = !rows && s.inner % V == 0 && (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
-            const void *kernel = rows      ? reinterpret_cast<const void *>(&axis_rows<T, FOLD>)
+            // Loads in flight per lane of a row: 16, but a row of few steps takes the registers for more warps (sums of 1000000
+            // x 65 floats: 198 us with 4, 257 with 8, 410 with 16; of 50000 x 700: 32, 28 and 31; of 30000 x 1500: 40,
+            // 35 and 33).
+            const void *by_rows = s.extent < 512    ? reinterpret_cast<const void *>(&axis_rows<T, FOLD, 4>)
+                                  : s.extent < 1500 ? reinterpret_cast<const void *>(&axis_rows<T, FOLD, 8>)
+                                                    : reinterpret_cast<const void *>(&axis_rows<T, FOLD, 16>);
+            const void *kernel = rows      ? by_rows
                                  : vectors ? reinterpret_cast<const void *>(&axis_columns<T, FOLD, V>)
                                            : reinterpret_cast<const void *>(&axis_columns<T, FOLD, 1>);
             const unsigned long long most = 1ull * ctx.sms * ctx.blocks_per_sm(kernel, 256, 0);  // blocks of 256
             unsigned long long want, cap;
             if (rows) {
-                // a warp per (row, piece): a wave of warps, in pieces of at least 2048 values
-                want = (8 * most + s.outer - 1) / s.outer;
-                cap = (s.extent + 2047) / 2048;
+                // a warp per (row, piece): a wave of warps in pieces of at least 2048 values, and four waves in pieces of at
+                // least 4096 (600 x 100000 floats: 57 -> 52 us)
+                const unsigned long long wave = 8 * most;
+                want = std::max(std::min((wave + s.outer - 1) / s.outer, (s.extent + 2047) / 2048),
+                                std::min((4 * wave + s.outer - 1) / s.outer, s.extent / 4096));
                 // a row per warp fills two thirds of a wave: no pieces, and no pass to fold them (5001 rows
-                // of 7003 floats: 35 + 4 us in pieces, 33 without)
-                if (s.outer * 3 >= 8 * most * 2) want = 1;
+                // of 7003 floats: 35 + 4 us in pieces, 33 without) -- unless the rows beyond the last full wave
+                // are less than a quarter of one and long, and would run alone (5001 x 100000: 389 us whole, 310 in
+                // four pieces; 7200 x 30000 doubles, 96 rows above two waves: 302 and 266)
+                if (s.outer * 3 >= wave * 2) {
+                    const bool alone = s.outer > wave && s.outer < 8 * wave && s.outer % wave * 4 < wave;
+                    want = alone ? std::min<unsigned long long>(4, s.extent / 4096) : 1;
+                }
+                cap = s.extent;
             } else {
-                // a thread per (o, piece, group of columns): four waves, in pieces of at least 64 values
+                // a thread per (o, piece, group of columns): four waves, in pieces of at least 64 values, at most 4096 of
+                // them, which one thread per output folds (1000000 x 65 floats: 9327 pieces 827 us, 4663 439)
                 const unsigned long long groups = s.outer * (vectors ? s.inner / V : s.inner);
-                want = (4 * most * 256 + groups - 1) / groups;
+                want = std::min<unsigned long long>((4 * most * 256 + groups - 1) / groups, 4096);
                 cap = (s.extent + 63) / 64;
             }
             s.pieces = want < cap ? want : cap;
@@ -199,7 +223,10 @@ namespace sci_cuda {
             }
             auto grid = [&](unsigned long long blocks) { return static_cast<unsigned>(blocks < most ? blocks : most); };
             if (rows) {
-                axis_rows<T, FOLD><<<grid((s.outer * s.pieces + 7) / 8), 256, 0, ctx.stream>>>(in, s, partial, out);
+                void *args[] = {&in, &s, &partial, &out};
+                if (int code = ctx.check(cudaLaunchKernel(kernel, dim3(grid((s.outer * s.pieces + 7) / 8)), dim3(256), args, 0, ctx.stream),
+                                         "launching an axis reduction"))
+                    return code;
             } else if (vectors) {
                 axis_columns<T, FOLD, V><<<grid((s.outer * s.pieces * (s.inner / V) + 255) / 256), 256, 0, ctx.stream>>>(in, s, partial, out);
             } else {
@@ -207,7 +234,7 @@ namespace sci_cuda {
             }
             if (int code = ctx.check(cudaGetLastError(), "launching an axis reduction")) return code;
             if (s.pieces > 1) {
-                axis_pieces<T><<<grid((s.outer * s.inner + 255) / 256), 256, 0, ctx.stream>>>(partial, s, out);
+                axis_pieces<T, FOLD><<<grid((s.outer * s.inner + 255) / 256), 256, 0, ctx.stream>>>(partial, s, out);
                 if (int code = ctx.check(cudaGetLastError(), "launching the axis piece fold")) return code;
             }
             return SCI_CUDA_OK;
