@@ -183,18 +183,33 @@ namespace sci_cuda {
         static constexpr int value = C::length <= 16 ? static_cast<int>(16 / sizeof(T)) : 1;
     };
 
-    // Blocks an SM holds of a short baked program: 64 registers a thread. The instructions' latency needs the warps: for
-    // exp(-a^2) sin b + log(1 + c^2) over 2^26 floats, 474 us with the 100 registers the compiler would
-    // take (two blocks), 409 with three, 387 with four; the program it replaces took 501.
-    template <class Program> struct GradientBlocks {
-        static constexpr int value = 1;
+    // Long float programs of many functions walk back guarded at once: with both walks such a kernel is bound by its
+    // instructions' way in (23 nodes, 8 of them functions, 421 us with both, 360 guarded; 28 nodes with none 190
+    // and 227, doubles of 23 nodes 571 either way).
+    template <typename T, class C> __host__ __device__ constexpr bool guarded_walk() {
+        int functions = 0;
+        for (int s = 0; s < C::length; ++s) functions += C::steps[s].code >= kRoot && C::steps[s].code < kAdd ? 1 : 0;
+        return sizeof(T) == 4 && C::length > 16 && functions > 6;
+    }
+
+    // Blocks an SM holds of a short baked program that runs and differentiates in one pass; 0: as the compiler takes it. The
+    // instructions' latency needs the warps as long as the program's values fit the registers that leaves (four blocks: 64,
+    // three: 80, two: 128). Over 2^24 floats with four, three and two blocks, us: exp(-a^2) sin b + log(1 + c^2), 8 nodes,
+    // 108, 113, 131; three quotients, 10 nodes, 206, 225, 247; a polynomial of 12 nodes 189, 149, 151; sines, cosines and a
+    // tangent, 14 nodes, 537, 354, 218. Doubles, which hold two elements a thread: 12 nodes 160, 171, 204; 13 nodes 330,
+    // 309, 317; 14 nodes 517, 522, 438. The two-pass form lost up to a fifth by such bounds and has none.
+    template <typename T, class Program, int FORM> struct GradientBlocks {
+        static constexpr int value = 0;
     };
-    template <class C> struct GradientBlocks<Baked<C>> {
-        static constexpr int value = C::length <= 16 ? 4 : 1;
+    template <typename T, class C> struct GradientBlocks<T, Baked<C>, kGradRecompute> {
+        static constexpr int value = C::length > 16                          ? 0
+                                     : C::length <= (sizeof(T) == 4 ? 11 : 12) ? 4
+                                     : C::length <= 13                         ? 3
+                                                                               : 2;
     };
 
     template <typename T, class Program, int FORM>
-    __global__ void __launch_bounds__(256, GradientBlocks<Program>::value) gradient_stream(const __grid_constant__ GradientLaunch<T> L) {
+    __global__ void __launch_bounds__(256, GradientBlocks<T, Program, FORM>::value) gradient_stream(const __grid_constant__ GradientLaunch<T> L) {
         constexpr int E = GradientWidth<T, Program>::value;
         constexpr bool forward = FORM != kGradReplay, backward = FORM != kGradRecord;
         const unsigned long long count = L.count;
@@ -391,7 +406,8 @@ namespace sci_cuda {
                         }
                         return lost;
                     };
-                    if (reverse(Int<1>{})) reverse(Int<0>{});
+                    if constexpr (guarded_walk<T, C>()) reverse(Int<0>{});
+                    else if (reverse(Int<1>{})) reverse(Int<0>{});
 #pragma unroll
                     for (int a = 0; a < C::arguments; ++a) {
                         T *dst = L.gradients[a];
