@@ -77,8 +77,7 @@ namespace sci_cuda {
         std::string name;
 
         ReduceState *state{nullptr};   // reduction scratch (device)
-        double *result{nullptr};       // device: a spare double, with the status word 8 bytes on
-        int *status{nullptr};          // device-side error word (in result's allocation)
+        int *status{nullptr};          // device-side error word
         double *host_result{nullptr};  // pinned, with host_status 8 bytes on: blocking reductions write both
         int *host_status{nullptr};     // pinned (in host_result's allocation)
         unsigned *notice_word{nullptr};  // pinned (in host_result's allocation): the last reduction's notice
@@ -136,9 +135,8 @@ namespace sci_cuda {
             return occupancy[key];
         }
 
-        // Reads and clears the device error word; waits for the stream. status_queued: a copy of the
-        // status word into host_status is already queued on the stream.
-        int drain(bool status_queued = false);
+        // Reads and clears the device error word; waits for the stream.
+        int drain();
 
         // The notice of the next blocking reduction, and the wait for the last one handed out: its result and the status
         // word are then in host_result and host_status. The host polls the word for a while, then
@@ -201,9 +199,9 @@ namespace sci_cuda {
     // kernel's static part (mbarriers, fold scratch) is under 4 KB.
     constexpr size_t kChunkSharedOptIn = 44 * 1024;
 
-    // The context's reduction result (a double) and status word (an int after it), one allocation.
+    // A blocking reduction's result (a double) and status word (an int after it) on the host; the notice's
+    // word follows, in a 16-byte piece of its own.
     constexpr size_t kResultBytes = 16;
-    // On the host the notice's word follows, in a 16-byte piece of its own.
     constexpr size_t kHostResultBytes = 32;
 
     // The generic interpreter's kernels, compiled ahead of time (chunk_kernels_f32.cu / _f64.cu).

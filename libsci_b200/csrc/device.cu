@@ -26,10 +26,9 @@ using namespace sci_cuda;
 
 namespace sci_cuda {
 
-    int Context::drain(bool status_queued) {
-        int code = status_queued ? SCI_CUDA_OK
-                                 : check(cudaMemcpyAsync(host_status, status, sizeof(int), cudaMemcpyDeviceToHost, stream),
-                                         "reading the device status");
+    int Context::drain() {
+        int code = check(cudaMemcpyAsync(host_status, status, sizeof(int), cudaMemcpyDeviceToHost, stream),
+                         "reading the device status");
         if (code) return code;
         code = check(cudaStreamSynchronize(stream), "synchronizing the stream");
         if (code) return code;
@@ -281,13 +280,11 @@ int sci_cuda_open(uint32_t ordinal, sci_cuda_context **context) {
     int least = 0, greatest = 0;
     cudaDeviceGetStreamPriorityRange(&least, &greatest);
     if (cudaStreamCreateWithPriority(&ctx->stream, cudaStreamNonBlocking, greatest) != cudaSuccess) return SCI_CUDA_ERROR_DEVICE;
-    // the reduction's result with the status word after it (device and pinned host): a blocking
-    // reduction reads both with one copy
-    if (cudaMalloc(&ctx->state, sizeof(ReduceState)) != cudaSuccess || cudaMalloc(&ctx->result, kResultBytes) != cudaSuccess ||
+    // a blocking reduction's result, the status word after it and the notice's word, in pinned host memory
+    if (cudaMalloc(&ctx->state, sizeof(ReduceState)) != cudaSuccess || cudaMalloc(&ctx->status, sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&ctx->host_result, kHostResultBytes) != cudaSuccess) {
         return SCI_CUDA_ERROR_MEMORY;
     }
-    ctx->status = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(ctx->result) + sizeof(double));
     ctx->host_status = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(ctx->host_result) + sizeof(double));
     cudaMemsetAsync(ctx->state, 0, sizeof(ReduceState), ctx->stream);
     cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream);
@@ -323,7 +320,7 @@ int sci_cuda_close(sci_cuda_context *context) {
         }
         context->retired.clear();
         cudaFree(context->state);
-        cudaFree(context->result);  // and the status word
+        cudaFree(context->status);
         cudaFree(context->sweep_flags);
         if (context->side) cudaStreamDestroy(context->side);
         if (context->side_done) cudaEventDestroy(context->side_done);
