@@ -36,3 +36,9 @@ def device():
     dev = Device(0)
     yield dev
     dev.close()
+
+
+def pytest_collection_modifyitems(items):
+    """The integration programs, which fail where the reference sources they are compiled from were absent at
+    build time, come last: a run that stops at the first failure has then run every other test."""
+    items.sort(key=lambda item: item.path.name == "test_integration_gpu.py")
