@@ -30,8 +30,8 @@
 // What bounds it: the chain of columns (700 cycles each at order 128, 790 at 256: two barriers, a
 // warp-wide maximum and vote, four trips through shared memory) and of barriers; systems of order 152
 // or less run several to an SM and fill each other's gaps. 4096 systems with orders uniform in
-// [8, 256]: 2.81 ms, where a column by column elimination in shared memory (about 3900 cycles a
-// column at 256) took 11.8 ms. One wave of 148 systems of order 64 / 128 / 256: 49 / 98 / 248 us.
+// [8, 256]: 2.94 ms, where a column by column elimination in shared memory (about 3900 cycles a
+// column at 256) took 11.8 ms. One wave of 148 systems of order 64 / 128 / 256: 41 / 101 / 254 us.
 #pragma once
 
 #include "chunk_kernel.cuh"  // static_for

@@ -22,7 +22,7 @@ def system(n, width, zeros, seed):
     return a, b
 
 
-def judge(a, b, x, error, iterations):
+def verify(a, b, x, error, iterations):
     for j in range(b.shape[1]):
         if b[:, j].any():
             assert backward_error(a, b[:, j], x[:, j]) <= 1e-14, j
@@ -36,7 +36,7 @@ def test_solves(device, width, zeros):
     for n in ORDERS:
         a, b = system(n, width, zeros, n)
         x, error, iterations = device.solve(device.array(a.ravel()), device.array(b.ravel()), n, width, refine=True)
-        judge(a, b, x.numpy().reshape(n, width), error, iterations)
+        verify(a, b, x.numpy().reshape(n, width), error, iterations)
 
 
 @pytest.mark.parametrize("width,zeros", [(1, [0]), (3, [1]), (8, [0, 5])])
@@ -45,8 +45,8 @@ def test_adjoints(device, width, zeros):
         a, b = system(n, width, [], n)
         g = system(n, width, zeros, n + 1)[1]
         x, _, db, error, iterations = device.solve_gradient(*(device.array(v.ravel()) for v in (a, b, g)), n, width, refine=True)
-        judge(a, b, x.numpy().reshape(n, width), error, iterations)
-        judge(a.T, g, db.numpy().reshape(n, width), error, iterations)
+        verify(a, b, x.numpy().reshape(n, width), error, iterations)
+        verify(a.T, g, db.numpy().reshape(n, width), error, iterations)
 
 
 def test_batch(device):
@@ -58,5 +58,5 @@ def test_batch(device):
     batch = device.solve_batch(orders, *[[v.pointer for v in t] for t in (da, db, dx)], errors, iterations)
     batch.launch()
     for k, n in enumerate(orders):
-        judge(a[k], b[k], dx[k].numpy().reshape(n, 1), errors.numpy()[k], iterations.numpy()[k])
+        verify(a[k], b[k], dx[k].numpy().reshape(n, 1), errors.numpy()[k], iterations.numpy()[k])
     batch.close()
